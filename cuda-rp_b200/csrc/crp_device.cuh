@@ -14,6 +14,7 @@
 #pragma once
 #include <cuda_pipeline.h>
 
+#include <cmath>
 #include <cstdint>
 
 namespace crp {
@@ -73,6 +74,10 @@ struct GridParams {
 struct BubbleParams {
   double PL0, T0, gam, sig, mu, rho, K0, dt0;
   double inv_rho;  // 1 / rho
+  // Constants of the FP64 thermal model and gas pressure (thermal64,
+  // rp_substep_full): 3 gam, 3 gam rho, -2 sigma rho, 4.5 gam (gam - 1),
+  // 1.5 (gam - 1), 0.75 gam, gam / (2 (gam - 1) T0 K0), 3 (gam - 1) K0.
+  double th_g3, th_g3rho, th_base, th_km, th_h, th_kl, th_ca, k0g;
   // Smallest |a|^2 whose square root exceeds 0.1 in FP64 / FP32: the series
   // switch of Upsilon and Lp (cabs(a) > 0.1) without a square root on the
   // sub-step's critical path, deciding exactly as the square root would.
@@ -85,6 +90,32 @@ struct BubbleParams {
   double rk_rtol;  // relative tolerance of the rk45 scheme
   int reuse;       // ext.rp_reuse: keep a bubble's last solve of the step while its gathered pressure is unchanged
 };
+
+// The derived constants of a BubbleParams whose physical ones are set.
+inline void derive_bubble_constants(BubbleParams& b) {
+  b.inv_rho = 1.0 / b.rho;
+  b.th_g3 = 3.0 * b.gam;
+  b.th_g3rho = 3.0 * b.gam * b.rho;
+  b.th_base = -2.0 * b.sig * b.rho;
+  b.th_km = 4.5 * b.gam * (b.gam - 1.0);
+  b.th_h = 1.5 * (b.gam - 1.0);
+  b.th_kl = 0.75 * b.gam;
+  b.th_ca = b.gam / (2.0 * (b.gam - 1.0) * b.T0 * b.K0);
+  b.k0g = 3.0 * (b.gam - 1.0) * b.K0;
+  double c = 0.01;
+  while (std::sqrt(c) > 0.1) c = std::nextafter(c, 0.0);
+  while (!(std::sqrt(c) > 0.1)) c = std::nextafter(c, 1.0);
+  b.abs2_cut64 = c;
+  float cf = 0.01f;
+  while (std::sqrt(cf) > 0.1f) cf = std::nextafter(cf, 0.0f);
+  while (!(std::sqrt(cf) > 0.1f)) cf = std::nextafter(cf, 1.0f);
+  b.abs2_cut32 = cf;
+  b.rho32 = (float)b.rho;
+  b.sig32 = (float)b.sig;
+  b.mu32 = (float)b.mu;
+  b.gam32 = (float)b.gam;
+  b.inv_rho32 = (float)b.inv_rho;
+}
 
 // Default relative tolerance of the rk45 scheme (ext.rp_tol = 0).
 constexpr double kRk45DefaultTol = 1.0e-6;
@@ -281,9 +312,11 @@ __device__ __forceinline__ double p0_at(const GridParams& g, const S& px, const 
 
 // ---------------------------------------------------------------------------
 // Bubble physics (inc/bubble_CUDA_kernel.cuh:227-340, inc/complex.cuh).  The
-// thermal model (alpha_N, Upsilon, omega_N, Lp_N) is a template on the real
-// type: FP64 for the FP64 path, FP32 for the mixed path.  The radius update,
-// its step-size control and the gas-pressure update stay FP64 in both.
+// thermal model (alpha_N, Upsilon, omega_N, Lp_N) comes in two forms: a template on
+// the real type in the reference's coth form, for the rk45 scheme, the reference
+// scheme with the temperature branch and the mixed path near equilibrium; and
+// thermal64 for the reference scheme elsewhere.  The radius update, its step-size
+// control and the gas-pressure update stay FP64.
 template <typename R>
 struct Cx {
   R re, im;
@@ -514,6 +547,262 @@ __device__ __forceinline__ void rp_substep(double& Rt, double& Rp, double& Rn, d
     Rt = (1.0 + qr) * Rn - qr * Rm + (dtp * inv_Rn) * (0.5 * (dtp + dtm) * acc);
   }
   remain -= dtp;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 thermal model of the reference radius scheme without the temperature
+// branch.
+
+// 1 / x, x^(-1/2) and x^(-1/4) of normal numbers (the roots: positive ones)
+// without the branches of the general operators: a hardware seed (at least 20
+// correct bits, PTX rcp/rsqrt.approx.ftz.f64) and one step of Householder's
+// third-order iteration (relative error e of the seed -> e^3, then the rounding
+// of the last operations: recip within 1.0, sqrt_pos within 1.5 units of 2^-53,
+// measured over 7e7 values).  Latency 40 and 50 cycles against 75 and 95 of the
+// operators, and as straight-line code the chains of a sub-step overlap.
+__device__ __forceinline__ double recip(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+// a / b, with the residual of the first quotient added: rounded as a division is
+// (but for rare ties of the last bit).
+__device__ __forceinline__ double quotient(double a, double b) {
+  const double y = recip(b), q = a * y;
+  return fma(fma(-q, b, a), y, q);
+}
+__device__ __forceinline__ double rsqrt_seed(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rsqrt_pos(double x) {
+  const double y = rsqrt_seed(x);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double sqrt_pos(double x) {
+  const double y = rsqrt_seed(x);
+  const double s = x * y;
+  const double e = fma(-s, y, 1.0);
+  return fma(s * e, fma(0.375, e, 0.5), s);
+}
+__device__ __forceinline__ double rroot4_pos(double x) {
+  const double r = rsqrt_seed(x);
+  const double y = r * rsqrt_seed(r), y2 = y * y;
+  const double e = fma(-(x * y2), y2, 1.0);
+  return fma(y * e, fma(0.15625, e, 0.25), y);
+}
+// The larger and the smaller of two numbers; b where a is NaN.
+__device__ __forceinline__ double larger(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ double smaller(double a, double b) { return a < b ? a : b; }
+
+// Per-bubble constants of the FP64 radius solve: PG0 R0^3 and T0 / (PG0 R0^3)
+// (init_bub_params, src/bubble_CUDA.cu:666-670, PG0 = PL0 + 2 sigma / R0).
+struct BubbleConst {
+  double pgr, tpgr;
+};
+__device__ __forceinline__ BubbleConst bubble_const(const BubbleParams& b, double R0) {
+  const double pgr = (b.PL0 + 2.0 * b.sig / R0) * (R0 * R0 * R0);
+  return {pgr, b.T0 / pgr};
+}
+
+// The thermal model's functions of a = alpha_N = s (1 + i).  a^2 = i w with
+// w = 2 s^2 real; with c = a coth(a) - 1 and
+//   T = (a^2 - 3 c) / (a^2 c)
+// both functions follow without cancellation:
+//   Upsilon = 3 gam (3 + i w T) / (3 gam + i w T) (:297-307),  Lp = R T (:310-323).
+// T has Gauss's continued fraction 1 / (5 + a^2 / (7 + a^2 / (9 + ...)))
+// (Lambert's fraction of tanh without its first two levels).  Its 16th
+// convergent is the quotient A / B of polynomials in i w of degrees 7 and 8
+// with real coefficients; it is within 1e-17 of T for w < 32 (s < 4).  Real and
+// imaginary parts are the even and odd powers: A = Ar + i w Aj, B = Br + i w Bj
+// with four polynomials in -w^2, 13 multiply-adds together, against an
+// exponential, a sine and cosine and the complex products of the coth form.
+// Measured against 60 digits (s = 0.02 to 4.5): T within 5e-16, its imaginary part
+// within 2e-15; the coth form lost up to 3e-11 and 4e-8 for s < 0.5 and needed a
+// series below |a| = 0.1.
+// The 36th convergent (degrees 17 and 18, 33 multiply-adds) is within 1e-17 of T up
+// to w = 760 (s = 19.5), and from there coth(a) = 1 in FP64.  Between 32 and 760 T is
+// within 3e-15 and its imaginary part within 4e-15 (rounding of the alternating
+// sums); the coth form's exponential, sine and cosine took 930 cycles an evaluation there.
+constexpr double kThermalCut2 = 32.0 * 32.0;
+constexpr double kThermalLarge2 = 760.0 * 760.0;
+static __constant__ double kThermalA16[8] = {1.0 / 5.0, 2.0 / 175.0, 26.0 / 121275.0, 4.0 / 2255715.0,
+                                             2.0 / 283468185.0, 4.0 / 300678753375.0, 4.0 / 383365410553125.0,
+                                             8.0 / 3518144372646028125.0};
+static __constant__ double kThermalB16[9] = {1.0, 3.0 / 35.0, 13.0 / 5775.0, 26.0 / 1025325.0, 1.0 / 7268415.0,
+                                             2.0 / 5466886425.0, 2.0 / 4510181300625.0,
+                                             4.0 / 20573943699684375.0, 1.0 / 73881031825566590625.0};
+static __constant__ double kThermalA36[18] = {
+    1.0 / 5.0, 34.0 / 2625.0, 176.0 / 574875.0, 992.0 / 269386425.0, 899.0 / 34519946175.0, 58.0 / 494195810625.0,
+    116.0 / 327651822444375.0, 8.0 / 10851362135420625.0, 1.0 / 926706326364921375.0, 2.0 / 1787031215351808118875.0,
+    8.0 / 9736692136585954530046875.0, 16.0 / 37868777631221801725789453125.0,
+    2.0 / 13431764127504902135201166796875.0, 4.0 / 115444547392545269680912006673671875.0,
+    8.0 / 1597098350144268775855630337659134609375.0, 16.0 / 39408401789809832044237678581739146486328125.0,
+    1.0 / 65614988980033370353655734838595678899736328125.0,
+    2.0 / 11847245565267885250945018515252319995099692197265625.0};
+static __constant__ double kThermalB36[19] = {
+    1.0, 7.0 / 75.0, 187.0 / 63875.0, 5456.0 / 122448375.0, 7192.0 / 18587663325.0, 899.0 / 428303035875.0,
+    29.0 / 3854727322875.0, 116.0 / 6282367552085625.0, 1.0 / 31520623345745625.0, 1.0 / 25899003121040697375.0,
+    1.0 / 29959052727956783169375.0, 8.0 / 392713249508966832711890625.0, 4.0 / 463164280258789728800040234375.0,
+    2.0 / 809569056048704555967124871484375.0, 2.0 / 4399719972849225277839202032118828125.0,
+    8.0 / 160850619550244212425459912578527128515625.0, 1.0 / 354675616108288488398139107235652318376953125.0,
+    1.0 / 15988185648134797909507447389004480425235751953125.0,
+    1.0 / 4371633613583849657598711832128106078191786420791015625.0};
+
+struct ThermalRatio {
+  double Ar, Aj, Br, Bj;  // T = (Ar + i w Aj) / (Br + i w Bj)
+};
+// c[first] + c[first + 2] x + c[first + 4] x^2 + ... over the n coefficients of c.
+template <int N>
+__device__ __forceinline__ double every_other(const double (&c)[N], int first, double x) {
+  int k = N - 1 - ((N - 1 - first) & 1);
+  double v = c[k];
+#pragma unroll
+  for (k -= 2; k >= first; k -= 2) v = fma(v, x, c[k]);
+  return v;
+}
+template <int N, int M>
+__device__ __forceinline__ ThermalRatio thermal_convergent(const double (&a)[N], const double (&b)[M], double w2) {
+  const double x = -w2;
+  return {every_other(a, 0, x), every_other(a, 1, x), every_other(b, 0, x), every_other(b, 1, x)};
+}
+__device__ __forceinline__ ThermalRatio thermal_ratio16(double w2) {
+  return thermal_convergent(kThermalA16, kThermalB16, w2);
+}
+__device__ __forceinline__ ThermalRatio thermal_ratio36(double w2) {
+  return thermal_convergent(kThermalA36, kThermalB36, w2);
+}
+// coth(a) = 1: T = (a^2 - 3 c) / (a^2 c) with c = a - 1, both times w.
+__device__ __forceinline__ ThermalRatio thermal_ratio_large(double w2) {
+  const double w = sqrt_pos(w2), s = sqrt_pos(0.5 * w);
+  return {-3.0 * w * (s - 1.0), w - 3.0 * s, -w2 * s, w * (s - 1.0)};
+}
+
+// omega_N and Lp of a bubble of radius Rb in the form the gas-pressure update
+// uses: (Re Lp, Im Lp) / |Lp|^2 = (lr, li) / den.
+struct Thermal {
+  double omega, lr, li, den;
+};
+
+// solveOmegaN (:263-288) and solveLp (:310-323) in FP64.  The gas pressure
+// cancels in omega_N (its coefficients 1 / (PG x^3) and PG enter as a product
+// only), so the model depends on Rb alone.  The iteration runs on
+// eta = (omega rho Rb)^2: w^2 = (2 coeff_alpha omega / Rb)^2 is proportional to it, T
+// depends on w^2, and Im(Upsilon) / (4 omega) on Im(Upsilon) / w, so each of the
+// three rounds takes one reciprocal and no square root.
+struct ThermalPre {
+  double base, c3, gq, ws2, caQ;
+};
+__device__ __forceinline__ ThermalPre thermal_pre(const BubbleParams& b, double pgr, double inv_Rb, double& eta) {
+  const double iR2 = inv_Rb * inv_Rb;
+  const double Q = pgr * iR2 * inv_Rb;  // PG0 / x^3
+  const double caR = b.th_ca * pgr * inv_Rb;
+  const double ws = 2.0 * caR * (b.inv_rho * inv_Rb);
+  ThermalPre t;
+  t.base = b.th_base * inv_Rb;  // -2 sigma rho / Rb
+  t.c3 = 4.0 * iR2;
+  t.gq = b.th_g3rho * Q;
+  t.ws2 = ws * ws;
+  t.caQ = caR * Q;
+  eta = larger(t.gq + t.base - b.mu * b.mu * t.c3, 1.0e-6 * 2.22044604925031308e-016);
+  return t;
+}
+// eta from Re(Upsilon) / (3 gam) and the effective viscosity.
+__device__ __forceinline__ double thermal_eta(const ThermalPre& t, double ur, double mu_eff) {
+  return larger(fma(t.gq, ur, fma(-(mu_eff * t.c3), mu_eff, t.base)), 1.0e-6 * 2.22044604925031308e-016);
+}
+__device__ __forceinline__ double thermal_round(const BubbleParams& b, const ThermalPre& t, const ThermalRatio& r,
+                                                double w2) {
+  const double p = -w2 * r.Aj;
+  const double dr = fma(b.th_g3, r.Br, p), nr = fma(3.0, r.Br, p);
+  const double di = fma(b.th_g3, r.Bj, r.Ar), ni = fma(3.0, r.Bj, r.Ar);
+  const double w2di = w2 * di;
+  const double inv = recip(fma(w2di, di, dr * dr));
+  const double mu_eff = fma(b.th_km * t.caQ * fma(r.Ar, r.Br, -p * r.Bj), inv, b.mu);
+  return thermal_eta(t, fma(w2di, ni, nr * dr) * inv, mu_eff);
+}
+__device__ __forceinline__ Thermal thermal_result(const BubbleParams& b, const ThermalPre& t, const ThermalRatio& r,
+                                                  double eta, double w2, double Rb, double inv_Rb) {
+  Thermal o;
+  o.omega = b.inv_rho * inv_Rb * sqrt_pos(eta);
+  o.lr = fma(r.Ar, r.Br, w2 * (r.Aj * r.Bj));
+  o.li = sqrt_pos(w2) * fma(r.Aj, r.Br, -r.Ar * r.Bj);
+  o.den = Rb * fma(r.Ar, r.Ar, w2 * (r.Aj * r.Aj));
+  return o;
+}
+// Any w, out of line: a bubble whose evaluations fall on both sides of a limit
+// of thermal64.
+static __device__ __noinline__ void thermal_any(const BubbleParams& b, double pgr, double Rb, double inv_Rb,
+                                                Thermal* o) {
+  double eta;
+  const ThermalPre t = thermal_pre(b, pgr, inv_Rb, eta);
+  double w2 = t.ws2 * eta;
+#pragma unroll 1
+  for (int k = 0;; k++) {
+    const ThermalRatio r = w2 < kThermalLarge2 ? thermal_ratio36(w2) : thermal_ratio_large(w2);
+    if (k == 3) {
+      *o = thermal_result(b, t, r, eta, w2, Rb, inv_Rb);
+      return;
+    }
+    eta = thermal_round(b, t, r, w2);
+    w2 = t.ws2 * eta;
+  }
+}
+// Three ranges in line, by the first w: a quiet bubble (w < 32: radii up to
+// about 20 um at rest), a compressed one, and a collapsed one (w >= 760), each valid
+// while all of its evaluations stay inside.  With coth(a) = 1 and d = 1 / s:
+// c / a^2 = (d - i d (1 - d)) / 2, and Lp's parts are polynomials in d.
+__device__ __forceinline__ Thermal thermal64(const BubbleParams& b, double pgr, double Rb, double inv_Rb) {
+  double eta;
+  const ThermalPre t = thermal_pre(b, pgr, inv_Rb, eta);
+  double w2 = t.ws2 * eta;
+  Thermal o;
+  if (w2 < kThermalCut2) {
+    bool in = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      eta = thermal_round(b, t, thermal_ratio16(w2), w2);
+      w2 = t.ws2 * eta;
+      in = in && w2 < kThermalCut2;
+    }
+    o = thermal_result(b, t, thermal_ratio16(w2), eta, w2, Rb, inv_Rb);
+    if (in) return o;
+  } else if (w2 < kThermalLarge2) {
+    bool in = true;
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) {
+      eta = thermal_round(b, t, thermal_ratio36(w2), w2);
+      w2 = t.ws2 * eta;
+      in = in && w2 < kThermalLarge2;
+    }
+    o = thermal_result(b, t, thermal_ratio36(w2), eta, w2, Rb, inv_Rb);
+    if (in) return o;
+  } else {
+    bool in = true;
+    double d = rroot4_pos(0.25 * w2);
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) {
+      const double h = b.th_h * d, dr = 1.0 + h, di = fma(-h, d, h);
+      const double inv = recip(fma(di, di, dr * dr));
+      const double mu_eff = fma(b.th_kl * t.caQ * (d * d) * di, inv, b.mu);
+      eta = thermal_eta(t, dr * inv, mu_eff);
+      w2 = t.ws2 * eta;
+      in = in && w2 >= kThermalLarge2;
+      d = rroot4_pos(0.25 * w2);
+    }
+    o.omega = b.inv_rho * inv_Rb * sqrt_pos(eta);
+    const double e = 1.0 - d, f = fma(-3.0, d, 2.0), de = d * e;
+    o.lr = 4.0 * e;
+    o.li = fma(fma(fma(6.0, d, -12.0), d, 12.0), d, -4.0);
+    o.den = Rb * d * fma(9.0 * de, de, f * f);
+    if (in) return o;
+  }
+  Thermal u;
+  thermal_any(b, pgr, Rb, inv_Rb, &u);
+  return u;
 }
 
 // Smooth delta (inc/bubble_CUDA_kernel.cuh:214-222), band 2 (the only band

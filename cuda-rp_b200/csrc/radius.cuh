@@ -6,18 +6,68 @@
 
 namespace crp {
 
-// Per-bubble state of BubbleRadiusKernel (inc/bubble_CUDA_kernel.cuh:471-554)
-// while its sub-steps run.
-struct RpState {
-  double Rt, Rp, Rn, d1Rp, PGp, dtL, remain, time, PC0, PC1, PC2, heat, vis, re_n;
-  BubbleR0 r;
-  long long count;
+// The sub-step comes in two forms of the same scheme:
+//   kLean  the thermal model of thermal64, no divisions but reciprocals;
+//   kHeat  the reference's operation order with the coth form, kept for runs with the
+//          temperature branch.  A resting bubble's heat flux is what the rounding of
+//          its gas pressure leaves (the gas pressure has a fixed point at which
+//          PG0 R0^3 and PG R^3 differ by rounding), so another order of operations
+//          moves the temperature field by up to 1e-8 before the burst arrives; with
+//          the order kept it is reproduced to the bit.
+enum RadiusForm { kLean = 0, kHeat = 1 };
+
+// Per-bubble constants of the lean form: the mixed path (T = float) also keeps
+// the FP32 thermal model's.
+template <typename T>
+struct RadiusConst {
+  BubbleConst c;
+};
+template <>
+struct RadiusConst<float> {
+  BubbleConst c;
+  double R0;
+  ThermalConst<float> f;
+};
+template <typename T, int FORM>
+struct RadiusConstOf {
+  using type = RadiusConst<T>;
+};
+template <typename T>
+struct RadiusConstOf<T, kHeat> {
+  using type = BubbleR0;
 };
 
+// Per-bubble state of BubbleRadiusKernel (inc/bubble_CUDA_kernel.cuh:471-554)
+// while its sub-steps run.  T: type of the thermal model near equilibrium.
+template <typename T, int FORM>
+struct RpState {
+  double Rt, Rp, Rn, d1Rp, PGp, dtL, remain, time, PC0, PC1, PC2, heat, vis, re_n;
+  typename RadiusConstOf<T, FORM>::type r;
+  int count;
+};
+template <typename T, int FORM>
+__device__ __forceinline__ void radius_const(const BubbleParams& b, double R0, RpState<T, FORM>& s) {
+  if constexpr (FORM == kHeat) {
+    s.r = bubble_r0(b, R0);
+  } else {
+    s.r.c = bubble_const(b, R0);
+    if constexpr (sizeof(T) == sizeof(float)) {
+      s.r.R0 = R0;
+      s.r.f = thermal_const32(b, bubble_r0(b, R0));
+    }
+  }
+}
+
+// Relative radius excursion |R/R0 - 1| above which the mixed path evaluates
+// the thermal model in FP64: FP32 is accurate for the small oscillations of a
+// quiet bubble, and its rounding is amplified once the bubble is driven.
+constexpr double kThermalFp64Excursion = 1.0e-3;
+
+// ---- kHeat ------------------------------------------------------------------
 // One pass of the sub-step loop of BubbleRadiusKernel (:506-539).  T is the
 // real type of the thermal model (omega_N, alpha_N, Lp_N); everything else is FP64.
-template <typename T>
-__device__ __forceinline__ void thermal_model(const BubbleParams& bp, const RpState& s, double PGn, double& omega,
+template <typename T, typename STATE>
+__device__ __forceinline__ void thermal_model(const BubbleParams& bp, const STATE& s, double PGn, double& omega,
                                               C64& lp) {
   Cx<T> alpha_t;
   ThermalConst<T> c;
@@ -30,13 +80,8 @@ __device__ __forceinline__ void thermal_model(const BubbleParams& bp, const RpSt
   lp = C64{(double)lp_t.re, (double)lp_t.im};
 }
 
-// Relative radius excursion |R/R0 - 1| above which the mixed path evaluates
-// the thermal model in FP64: FP32 is accurate for the small oscillations of a
-// quiet bubble, and its rounding is amplified once the bubble is driven.
-constexpr double kThermalFp64Excursion = 1.0e-3;
-
 template <typename T>
-__device__ __forceinline__ void rp_substep_full(const BubbleParams& bp, RpState& s) {
+__device__ __forceinline__ void rp_substep_heat(const BubbleParams& bp, RpState<T, kHeat>& s) {
   const double PGn = s.PGp;
   const double PL = s.PC2 * s.time * s.time + s.PC1 * s.time + s.PC0;
   rp_substep(s.Rt, s.Rp, s.Rn, s.d1Rp, PGn, PL, s.dtL, s.remain, bp);
@@ -60,6 +105,108 @@ __device__ __forceinline__ void rp_substep_full(const BubbleParams& bp, RpState&
   // 4 pi Rp^2 (4 mu d1Rp / Rp) d1Rp dt, with Rp^2 / Rp cancelled.
   s.vis += 4.0 * bp.pi * Rp * 4.0 * bp.mu * s.d1Rp * s.d1Rp * s.dtL;
   s.count++;
+}
+
+// ---- kLean ------------------------------------------------------------------
+// The FP32 thermal model of the mixed path near equilibrium.
+__device__ __forceinline__ Thermal thermal32(const ThermalConst<float>& c, double PG, double Rb) {
+  Cx<float> alpha;
+  const float omega = omega_n<float>(alpha, (float)PG, (float)Rb, c);
+  const Cx<float> lp = lp_n<float>(alpha, (float)Rb, c.cut2);
+  const double lr = lp.re, li = lp.im;
+  return {(double)omega, lr, li, lr * lr + li * li};
+}
+
+// One pass of the sub-step loop of BubbleRadiusKernel (:506-539):
+// solveRayleighPlesset (:227-260), one variable sub-step of the three-level
+// scheme; the thermal model at the old radius; solvePG (:326-340), with c1, c2, c3
+// and the numerator multiplied by R omega |Lp|^2, so that Lp and the time step enter
+// without divisions of their own and the gas pressure costs one reciprocal; and
+// the heat flux (:521-527).
+//
+// Bound by the FP64 pipe in the quiet phase (64 % busy; the launch over 262,144
+// bubbles of 10 sub-steps takes 77 us, 178 us with the coth form) and by the latency of
+// this chain once a few bubbles are stiff (one sub-step alone on an SM: 1,080
+// cycles for w < 32, 1,450 to 1,630 above; the coth form 4,130 above).
+template <typename T>
+__device__ __forceinline__ void rp_substep_lean(const BubbleParams& b, RpState<T, kLean>& s) {
+  const double eps = 2.22044604925031308e-016;
+  const double PGn = s.PGp;
+  const double PL = s.PC2 * s.time * s.time + s.PC1 * s.time + s.PC0;
+  const double Rm = s.Rn, Rn = s.Rp, d1n = s.d1Rp;
+  const double inv_Rn = recip(Rn);
+  Thermal th;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (fabs(Rn - s.r.R0) > kThermalFp64Excursion * s.r.R0)
+      th = thermal64(b, s.r.c.pgr, Rn, inv_Rn);
+    else
+      th = thermal32(s.r.f, PGn, Rn);
+  } else {
+    th = thermal64(b, s.r.c.pgr, Rn, inv_Rn);
+  }
+  // Radius update.  The velocity and acceleration limits, 0.01 Rn / |d1R| and
+  // 0.1 Rn / sqrt(|acc|) (:238-241): each quotient is formed only where it is the
+  // smaller step, decided on the products (the squares for the second), so a
+  // quiet sub-step divides by neither.
+  const double acc =
+      (PGn - PL - 2.0 * b.sig * inv_Rn - 4.0 * b.mu * inv_Rn * d1n) * b.inv_rho - 1.5 * d1n * d1n;
+  const double dtm = s.dtL;
+  double dtp = smaller(1.01 * dtm, b.dt0);
+  const double ad = fabs(d1n), aa = fabs(acc);
+  if (ad > eps && 0.01 * Rn < dtp * ad) dtp = smaller(0.01 * Rn * recip(ad), dtp);
+  if (aa > eps) {
+    const double lim = 0.1 * Rn;
+    if (lim * lim < dtp * dtp * aa) dtp = smaller(lim * rsqrt_pos(aa), dtp);
+  }
+  // q and the products below round as the reference's do: the rounding of 1 + q is
+  // the same at every sub-step of a constant growth and acts on R as a small
+  // force, 1e-9 of a driven bubble's radius after 1000 mixture steps.
+  const double sum = dtm + dtp;
+  const double q = quotient(dtp, dtm);
+  const double inv3 = recip(dtm * dtp * sum);
+  const double Rp = (1.0 + q) * Rn - q * Rm + (dtp * inv_Rn) * (0.5 * sum * acc);
+  const double d1 =
+      (dtm * dtm * Rp + (-dtm * dtm + dtp * dtp) * Rn - dtp * dtp * Rm) * inv3 + (dtp * inv_Rn) * acc;
+  s.Rt = Rp;
+  double last = dtp;
+  if (dtp >= s.remain) {
+    last = s.remain;
+    const double qr = quotient(last, dtm);
+    s.Rt = (1.0 + qr) * Rn - qr * Rm + (last * inv_Rn) * (0.5 * (dtm + last) * acc);
+  }
+  s.remain -= last;
+  s.Rn = Rn;
+  s.Rp = Rp;
+  s.d1Rp = d1;
+  s.dtL = dtp;
+  s.time = s.time + dtp;
+  s.count++;
+  // Gas pressure.
+  const double k0 = b.k0g * s.r.c.tpgr;  // 3 (gam - 1) K0 T0 / (PG0 R0^3)
+  const double R = 0.5 * (Rp + Rn), R3 = R * R * R;
+  const double Rp3 = Rp * Rp * Rp, Rn3 = Rn * Rn * Rn;
+  const double wd = th.omega * th.den;
+  const double wh = th.omega * dtp * th.lr;
+  const double g = 0.5 * b.th_g3 * (Rp - Rn);
+  const double a3 = 0.5 * k0 * wh * R3;
+  const double wn = k0 * th.li;
+  const double c1 = wd * (R + g) + a3 - wn * Rp3;
+  const double c2 = wd * (R - g) - a3 - wn * Rn3;
+  const double PG = (c2 * PGn + k0 * wh * s.r.c.pgr) * recip(c1);
+  s.PGp = PG;
+  // Heat flux (off the chain to the next sub-step) and viscous work:
+  // 4 pi Rp^2 (4 mu d1R / Rp) d1R dt, with Rp^2 / Rp cancelled.
+  const double hx = wh * (s.r.c.pgr - 0.5 * (PG + PGn) * R3) + th.li * (PG * Rp3 - PGn * Rn3);
+  s.heat -= 4.0 * b.pi * Rp * Rp * b.K0 * (s.r.c.tpgr * hx * recip(wd));
+  s.vis += 4.0 * b.pi * Rp * 4.0 * b.mu * d1 * d1 * dtp;
+}
+
+template <typename T, int FORM>
+__device__ __forceinline__ void rp_substep_full(const BubbleParams& b, RpState<T, FORM>& s) {
+  if constexpr (FORM == kHeat)
+    rp_substep_heat<T>(b, s);
+  else
+    rp_substep_lean<T>(b, s);
 }
 
 }  // namespace crp

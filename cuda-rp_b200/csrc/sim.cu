@@ -719,13 +719,14 @@ __device__ __forceinline__ double gather_pl(const GridParams& g, const BubblePar
 // solve's needs no solve: every input of its solve is unchanged, so its stored
 // results are what the solve would write; returns false for it.  The set-up
 // runs either way (a branch around it costs the radius kernel registers).
-template <typename S>
+template <typename S, typename T, int FORM>
 __device__ __forceinline__ bool rp_begin(const GridParams& g, const BubbleParams& bp, const BubbleArrays& b,
-                                         const S& px, const S& py, double t_cur, int n, RpState& s, bool reuse) {
+                                         const S& px, const S& py, double t_cur, int n, RpState<T, FORM>& s,
+                                         bool reuse) {
   const double PLp = gather_pl(g, bp, b, px, py, t_cur, n);
   const bool same = reuse && __double_as_longlong(PLp) == __double_as_longlong(b.PL_p[n]);
   b.PL_p[n] = PLp;
-  s.r = bubble_r0(bp, b.R0[n]);
+  radius_const(bp, b.R0[n], s);
   const double dt = g.dt;
   s.Rt = b.R_t[n];
   s.Rp = b.R_pn[n];
@@ -753,8 +754,9 @@ __device__ __forceinline__ void store_contrib(const GridParams& g, const BubbleP
 // Results of BubbleRadiusKernel (:542-550), then the bubble's void-fraction
 // contribution to the four cells of its stencil (VoidFractionReverseLookupKernel,
 // :595-617), stored for the per-cell gather.
+template <typename T, int FORM>
 __device__ __forceinline__ void rp_end(const GridParams& g, const BubbleParams& bp, const BubbleArrays& b, int n,
-                                       const RpState& s) {
+                                       const RpState<T, FORM>& s) {
   const double dt = g.dt;
   b.R_t[n] = s.Rt;
   b.R_p[n] = s.Rp;
@@ -764,7 +766,7 @@ __device__ __forceinline__ void rp_end(const GridParams& g, const BubbleParams& 
   b.dt[n] = s.dtL;
   b.re[n] = s.remain;
   b.Q_B[n] = (s.heat + s.vis) / (dt - s.remain + s.re_n);
-  b.nsub[n] = (int)min(s.count, (long long)INT32_MAX);
+  b.nsub[n] = s.count;
   store_contrib(g, bp, b, n, s.Rt);
 }
 
@@ -818,7 +820,7 @@ __device__ __forceinline__ void count_kept(int& n, unsigned long long* reused) {
   }
 }
 
-template <typename P>
+template <typename P, int FORM>
 __global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P>()) bubble_rp(const __grid_constant__ GridParams g,
                                                         const __grid_constant__ BubbleParams bp, BubbleArrays b,
                                                         const typename P::S px, const typename P::S py,
@@ -827,7 +829,7 @@ __global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P>()) bubble_rp(cons
                                                         int* __restrict__ next, long long* __restrict__ substep_max,
                                                         int* __restrict__ err, const int* __restrict__ solved,
                                                         unsigned long long* __restrict__ reused) {
-  RpState s;
+  RpState<typename P::T, FORM> s;
   const double t_cur = tdev[1];
   const bool reuse = bp.reuse && *solved > 0;
   int n = -1;
@@ -857,11 +859,11 @@ __global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P>()) bubble_rp(cons
     if (!__any_sync(0xffffffffu, n >= 0 || !drained)) break;
     if (n >= 0) {
       if (s.remain > 0.0 && s.count < bp.step_cap) {
-        rp_substep_full<typename P::T>(bp, s);
+        rp_substep_full(bp, s);
       } else {
         if (s.remain > 0.0) atomicOr(err, 1);
         rp_end(g, bp, b, n, s);
-        worst = max(worst, s.count);
+        worst = max(worst, (long long)s.count);
         n = -1;
       }
     }
@@ -1818,13 +1820,7 @@ struct Sim {
       int dev = 0, sms = 0, per_sm = 0;
       CRP_CUDA(cudaGetDevice(&dev));
       CRP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      const bool rk = cfg.ext_rp_scheme == CRP_RP_RK45;
-      if (mixed)
-        CRP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, rk ? bubble_rk45<PrecMixed> : bubble_rp<PrecMixed>, kRpThreads, 0));
-      else
-        CRP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, rk ? bubble_rk45<PrecFP64> : bubble_rp<PrecFP64>, kRpThreads, 0));
+      CRP_CUDA(mixed ? radius_occupancy<PrecMixed>(&per_sm) : radius_occupancy<PrecFP64>(&per_sm));
       rp_grid_full = std::max(1, std::min(sms * std::max(per_sm, 1), (hs.nb + kRpThreads - 1) / kRpThreads));
       rp_grid = rp_grid_full;
       couple_graph_grid = 4 * sms;
@@ -1970,24 +1966,8 @@ struct Sim {
     bp.sig = cfg.bub_sigma;
     bp.mu = cfg.bub_mu;
     bp.rho = cfg.bub_rho;
-    bp.inv_rho = 1.0 / cfg.bub_rho;
-    {
-      // Smallest squared modulus whose square root is above 0.1, per precision.
-      double c = 0.01;
-      while (std::sqrt(c) > 0.1) c = std::nextafter(c, 0.0);
-      while (!(std::sqrt(c) > 0.1)) c = std::nextafter(c, 1.0);
-      bp.abs2_cut64 = c;
-      float cf = 0.01f;
-      while (std::sqrt(cf) > 0.1f) cf = std::nextafter(cf, 0.0f);
-      while (!(std::sqrt(cf) > 0.1f)) cf = std::nextafter(cf, 1.0f);
-      bp.abs2_cut32 = cf;
-      bp.rho32 = (float)bp.rho;
-      bp.sig32 = (float)bp.sig;
-      bp.mu32 = (float)bp.mu;
-      bp.gam32 = (float)bp.gam;
-      bp.inv_rho32 = (float)bp.inv_rho;
-    }
     bp.K0 = cfg.bub_K0;
+    derive_bubble_constants(bp);
     bp.dt0 = d.bub_dt0;
     bp.pi = d.pi;
     bp.pi4r3 = d.pi4r3;
@@ -2821,19 +2801,24 @@ struct Sim {
     });
   }
 
+  // The radius kernel of this simulation: rk45, or the reference scheme in the
+  // form its temperature branch asks for (RadiusForm).
+  template <typename P>
+  auto radius_kernel() const {
+    return cfg.ext_rp_scheme == CRP_RP_RK45 ? bubble_rk45<P> : temperature_on ? bubble_rp<P, kHeat> : bubble_rp<P, kLean>;
+  }
+  template <typename P>
+  cudaError_t radius_occupancy(int* per_sm) const {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, radius_kernel<P>(), kRpThreads, 0);
+  }
   template <typename P>
   cudaError_t launch_rp() {
     using S = typename P::S;
     const S pxc = view<S>(px[cur_p]), pyc = view<S>(py[cur_p]);
-    if (cfg.ext_rp_scheme == CRP_RP_RK45)
-      return launch(kClassRp, [&] {
-        bubble_rk45<P><<<rp_grid, kRpThreads, 0, stream>>>(gp, bp, bub, pxc, pyc, d_scalars->t, lpt.order, d_next,
-                                                            d_substep_max, d_err, &d_scalars->loop,
-                                                            &d_scalars->reused);
-      });
+    const auto kernel = radius_kernel<P>();
     return launch(kClassRp, [&] {
-      bubble_rp<P><<<rp_grid, kRpThreads, 0, stream>>>(gp, bp, bub, pxc, pyc, d_scalars->t, lpt.order, d_next,
-                                                        d_substep_max, d_err, &d_scalars->loop, &d_scalars->reused);
+      kernel<<<rp_grid, kRpThreads, 0, stream>>>(gp, bp, bub, pxc, pyc, d_scalars->t, lpt.order, d_next, d_substep_max,
+                                                 d_err, &d_scalars->loop, &d_scalars->reused);
     });
   }
 

@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kRpThreads3) radius3(const __grid_constant__ G
                                                        const typename P::S pz, Scalars3* sc, int reuse,
                                                        const int* __restrict__ order) {
   const double dt = g.dt;
-  RpState s;
+  RpState<typename P::T, kLean> s;
   RkState r;
   int n = -1;
   bool drained = false;
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(kRpThreads3) radius3(const __grid_constant__ G
             r.PC2 = PC2;
             r.K = 3.0 * (bp.gam - 1.0) * bp.K0 * bp.T0 * r.r.inv_PG0;
           } else {
-            s.r = bubble_r0(bp, b.R0[n]);
+            radius_const(bp, b.R0[n], s);
             s.Rt = b.R_t[n];
             s.Rp = b.R_pn[n];
             s.Rn = b.R_nn[n];
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(kRpThreads3) radius3(const __grid_constant__ G
       worst = max(worst, r.count);
     } else {
       if (s.remain > 0.0 && s.count < bp.step_cap) {
-        rp_substep_full<typename P::T>(bp, s);
+        rp_substep_full(bp, s);
         continue;
       }
       if (s.remain > 0.0) atomicOr(&sc->err, 1);
@@ -638,9 +638,9 @@ __global__ void __launch_bounds__(kRpThreads3) radius3(const __grid_constant__ G
       b.dt[n] = s.dtL;
       b.re[n] = s.remain;
       b.Q_B[n] = (s.heat + s.vis) / (dt - s.remain + s.re_n);
-      b.nsub[n] = (int)min(s.count, (long long)INT32_MAX);
+      b.nsub[n] = s.count;
       contrib3(g, bp, b, n, s.Rt);
-      worst = max(worst, s.count);
+      worst = max(worst, (long long)s.count);
     }
     n = -1;
   }
@@ -1305,23 +1305,8 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
   bp.sig = c.bub_sigma;
   bp.mu = c.bub_mu;
   bp.rho = c.bub_rho;
-  bp.inv_rho = 1.0 / c.bub_rho;
-  {
-    double cc = 0.01;
-    while (std::sqrt(cc) > 0.1) cc = std::nextafter(cc, 0.0);
-    while (!(std::sqrt(cc) > 0.1)) cc = std::nextafter(cc, 1.0);
-    bp.abs2_cut64 = cc;
-    float cf = 0.01f;
-    while (std::sqrt(cf) > 0.1f) cf = std::nextafter(cf, 0.0f);
-    while (!(std::sqrt(cf) > 0.1f)) cf = std::nextafter(cf, 1.0f);
-    bp.abs2_cut32 = cf;
-    bp.rho32 = (float)bp.rho;
-    bp.sig32 = (float)bp.sig;
-    bp.mu32 = (float)bp.mu;
-    bp.gam32 = (float)bp.gam;
-    bp.inv_rho32 = (float)bp.inv_rho;
-  }
   bp.K0 = c.bub_K0;
+  derive_bubble_constants(bp);
   bp.dt0 = 0.1 * g.dt;
   bp.pi = pi;
   bp.pi4r3 = pi * 4.0 / 3.0;
