@@ -33,6 +33,7 @@ struct GridParams {
   double dt;
   double rho_inf, c_inf, P_inf;
   int pml_x0, pml_x1, pml_y0, pml_y1;
+  int px0, px1;  // cells i <= px0 and i >= px1 lie in the x PML
   int cyl;
   int plane_p, focused_p, plane_v, focused_v;
   int source_row;     // 0: ghost row y=0 when pml.y0 is off (reference); >0: forced row
@@ -226,6 +227,11 @@ struct F64 {
   __device__ __forceinline__ void put(K k, double v) const {
     p[k] = v;
   }
+  // Elements k and k + 1 (k even: one 16-byte access).
+  __device__ __forceinline__ double2 get2(unsigned k) const { return *reinterpret_cast<const double2*>(p + k); }
+  __device__ __forceinline__ void put2(unsigned k, double v, double w) const {
+    *reinterpret_cast<double2*>(p + k) = make_double2(v, w);
+  }
   // The value get() returns after put(v).
   __device__ static __forceinline__ double stored(double v) { return v; }
   // Asynchronous copy of element k into an 8-byte shared-memory slot, and the
@@ -247,6 +253,14 @@ struct F32c {
   __device__ __forceinline__ void put(K k, double v) const {
     const float h = (float)v;
     p[k] = make_float2(h, (float)(v - (double)h));
+  }
+  __device__ __forceinline__ double2 get2(unsigned k) const {
+    const float4 v = *reinterpret_cast<const float4*>(p + k);
+    return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+  }
+  __device__ __forceinline__ void put2(unsigned k, double v, double w) const {
+    const float h = (float)v, l = (float)w;
+    *reinterpret_cast<float4*>(p + k) = make_float4(h, (float)(v - (double)h), l, (float)(w - (double)l));
   }
   __device__ static __forceinline__ double stored(double v) {
     const float h = (float)v;
@@ -271,6 +285,13 @@ struct F32 {
   template <typename K>
   __device__ __forceinline__ void put(K k, double v) const {
     p[k] = (float)v;
+  }
+  __device__ __forceinline__ double2 get2(unsigned k) const {
+    const float2 v = *reinterpret_cast<const float2*>(p + k);
+    return make_double2((double)v.x, (double)v.y);
+  }
+  __device__ __forceinline__ void put2(unsigned k, double v, double w) const {
+    *reinterpret_cast<float2*>(p + k) = make_float2((float)v, (float)w);
   }
   __device__ static __forceinline__ double stored(double v) { return (double)(float)v; }
   template <typename K>

@@ -1,6 +1,6 @@
 // The fused FDTD pass on tiles staged by the tensor memory accelerator (TMA).
 //
-// Same arithmetic and output as the strip march of fdtd_strip (void-fraction
+// Same arithmetic and output as the march of fdtd_march (void-fraction
 // prediction, VelocityKernel with VelocityBoundaryKernel's faces and
 // MixturePressureKernel with its residual, inc/bubble_CUDA_kernel.cuh:622-867),
 // organised for latency hiding instead of a serial march: one thread per cell.

@@ -1,10 +1,10 @@
 // B200 implementation of CUDA-RP's simulation path behind the crp C ABI.
 //
 // One mixture time step (the main loop of solve_bubbles, src/bubble_CUDA.cu:206-285):
-//   fdtd_strip     fused: void-fraction prediction, velocity update with its
+//   fdtd_march     fused: void-fraction prediction, velocity update with its
 //                  boundary overrides (VelocityKernel, VelocityBoundaryKernel),
 //                  first pressure evaluation (MixturePressureKernel) and its
-//                  residual, one HBM pass in column strips
+//                  residual, one HBM pass
 //   vghost         velocity ghost cells (the rest of VelocityBoundaryKernel),
 //                  a launch of its own only without bubbles
 //   bubble_move    bubble state rotation (store_variables), velocity gather,
@@ -57,6 +57,16 @@ struct PrecMixed {
   using T = float;
 };
 
+// Values of the source's row for one step, by column i in [1, X]: the pressure
+// source at the step's start and end, and the velocity source at its end
+// (source_rows).  Evaluated ahead of the grid pass so that the pass carries no
+// transcendental code.
+struct SourceRows {
+  const double* p_prev;
+  const double* p_cur;
+  const double* v;
+};
+
 template <typename P>
 struct FdtdArgs {
   typename P::V vx_old, vy_old, vx_new, vy_new;
@@ -67,6 +77,13 @@ struct FdtdArgs {
   typename P::G fgC;       // f_gm of the previous step; receives the predicted f_g
   const double* tdev;  // {t_prev, t_cur} of this step, in device memory
   int rho_const;           // first step: the mixture density is still rho_inf everywhere
+  // Where the void fraction can be nonzero (fdtd_march): whether there are
+  // bubbles, and the support boxes {i0, j0, i1, j1} (empty when i0 > i1) of the last
+  // three steps, by value or (graph steps) in device memory.
+  int bubbles;
+  int supp[3][4];
+  const int* dsupp;
+  SourceRows src;
   unsigned long long* residual;
 };
 
@@ -102,7 +119,7 @@ __device__ __forceinline__ double face_q(const GridParams& g, double rhoa, doubl
 __device__ __forceinline__ double velocity_face_q(const GridParams& g, double v_old, double p0a, double p0b, double q,
                                                   double fa, double fb) {
   const double s2 = (-p0a + p0b) * g.rdx;  // rdx on both faces, as :661 and :671
-  return (v_old * fa - q * s2) * fb;
+  return fma(v_old, fa, -__dmul_rn(q, s2)) * fb;
 }
 
 // Split-pressure update of MixturePressureKernel (:856-859) for one component:
@@ -110,7 +127,7 @@ __device__ __forceinline__ double velocity_face_q(const GridParams& g, double v_
 // component's PML factors fa = 1 - s2, fb = 1 / (1 + s2) (as velocity_face).
 __device__ __forceinline__ double pressure_component(const GridParams& g, double pn, double fa, double fb, double s1,
                                                      double h) {
-  return pn * fa - g.s3p * (s1 + h) * fb;
+  return fma(pn, fa, -__dmul_rn(__dmul_rn(g.s3p, s1 + h), fb));
 }
 
 // s5 / 2 of :854: the void-fraction rate term; zero where f_g stays zero.
@@ -119,9 +136,8 @@ __device__ __forceinline__ double void_rate_half(const GridParams& g, double fg,
   return 0.5 * (-(fg - fgn) / g.dt / (1.0 - 0.5 * (fg + fgn)));
 }
 
-// The rarely taken parts of the strip update live in out-of-line functions so
-// that their transcendental code does not raise the register count of the
-// update loop.
+// The rarely taken parts of the tile kernel live in out-of-line functions so that
+// their transcendental code does not raise its register count.
 //
 // North face jf on the y0 face or the [ext] source row (VelocityBoundaryKernel
 // :734-798): v is the face from the update; pre receives the face before the
@@ -144,15 +160,6 @@ __device__ __noinline__ double vy_face_special(const GridParams& g, int jf, doub
 // North face jf of a column (VelocityKernel :668-676 with the y sections of
 // VelocityBoundaryKernel): y0 wall or source, [ext] source row, y1 wall.
 // q: dt / mean(rho) of the face (face_q).
-__device__ __forceinline__ double vy_face_value_f(const GridParams& g, int jf, double v_old, double p0a, double p0b,
-                                                  double q, double fa, double fb, double xm, double t_cur,
-                                                  double& pre) {
-  double v = velocity_face_q(g, v_old, p0a, p0b, q, fa, fb);
-  pre = v;
-  if ((jf == 0 && !g.pml_y0) || (g.source_row > 0 && jf == g.source_row)) v = vy_face_special(g, jf, v, xm, t_cur, &pre);
-  if (jf == g.f.Y && !g.pml_y1) v = 0.0;
-  return v;
-}
 __device__ __forceinline__ double vy_face_value(const GridParams& g, int jf, double v_old, double p0a, double p0b,
                                                 double q, double xm, double t_cur, double& pre) {
   double v = velocity_face_q(g, v_old, p0a, p0b, q, g.vay[jf + 1], g.vby[jf + 1]);
@@ -174,201 +181,12 @@ __device__ __noinline__ double source_row_pressure(const GridParams& g, double x
   return sv;
 }
 
-// One mixture step of the grid, fused: void-fraction prediction (store_variables,
-// src/bubble_CUDA.cu:1160-1162), VelocityKernel with VelocityBoundaryKernel's
-// faces (inc/bubble_CUDA_kernel.cuh:658-798), MixturePressureKernel with the
-// predicted void fraction (:816-867) and the residual of calculate_pressure_field.
-// The work is organised as column strips.  A warp holds the
-// 32 adjacent columns i = 30 s + lane of strip s and marches up a chunk of
-// kStripRows rows: lanes 1..30 update their cells, lanes 0 and 31 only provide
-// the values across the strip's edges.  Left/right neighbour values arrive by
-// warp shuffle, the row below stays in registers, so every array element is
-// read once per step (the two edge columns of a strip and the row under a
-// chunk once more, from L2), with 256-byte coalesced rows per warp load.  Rows
-// are staged through a per-warp ring of kStripStages rows in shared memory by
-// asynchronous copies issued kStripStages - 2 rows ahead, so each warp keeps
-// the next rows of all seven input arrays in flight while it computes.
-//
-// The kernel is bound by the latency of each row's dependent chain rather than
-// by bytes, so its instruction stream is kept short: element offsets are 32-bit
-// (the host rejects frames of 2^32 elements or more), one add per row; lanes
-// past the window stage a copy of column X+1 instead of branching around
-// their copies; only the stores are predicated.  The row loop stays rolled (an
-// unrolled chunk measured slower).
-constexpr int kStripCells = 30;
-constexpr int kStripWarps = 4;
-constexpr int kStripRows = 8;    // rows per chunk (measured best of 4-16 at 1024 x 2048)
-constexpr int kStripStages = 4;  // ring slots (rows) per warp; a smaller ring leaves more L1 (measured)
-constexpr int kStripFields = 7;  // pnx, pny, fgA, vx_old, vy_old, fgB, fgC
-
-template <typename P, int STAGES = kStripStages, int ROWS = kStripRows, int MINB = 4>
-__global__ void __launch_bounds__(32 * kStripWarps, MINB) fdtd_strip(const __grid_constant__ GridParams g,
-                                                               const FdtdArgs<P> a) {
-  using G = typename P::G;
-  using S = typename P::S;
-  using V = typename P::V;
-  __shared__ __align__(16) double ring[kStripWarps][STAGES][kStripFields][32];
-  const Frame& f = g.f;
-  const int X = f.X, Y = f.Y;
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x;
-  const int i = (blockIdx.x * kStripWarps + threadIdx.y) * kStripCells + lane;
-  const double t_prev = a.tdev[0], t_cur = a.tdev[1];
-  const bool inwin = i <= X + 1;                                 // column inside the window [0, X+1]
-  const bool cell = lane >= 1 && lane <= kStripCells && i <= X;  // updates cell (i, j)
-  const bool face = lane <= kStripCells && i <= X;               // east face F(i) needed
-  // Owner of the f_g prediction of this column.
-  const bool own = inwin && ((lane >= 1 && lane <= kStripCells) || (lane == 0 && i == 0) ||
-                             (lane == 31 && i == X + 1));
-  // Chunks are taken alternately from the bottom and the top of the grid, so
-  // that the PML bands at both y ends (the slowest chunks: general updates
-  // with divisions) start first and the cheap interior chunks fill the tail.
-  const int by = blockIdx.y, cy = (by & 1) ? (int)gridDim.y - 1 - (by >> 1) : (by >> 1);
-  const int j0 = 1 + cy * ROWS;
-  const int j1 = min(Y, j0 + ROWS - 1);
-  const double xm = ((double)i - 0.5) * g.dx;
-  const bool inner_col = i >= 1 && i <= X;
-  const bool src_rows = g.source_row > 0 && src_pressure(g);
-  // Offset of element (min(i, X+1), j0 - 1 + rr) is kb + rr * pitch.
-  const unsigned pitch = (unsigned)f.pitch;
-  const unsigned kb = (unsigned)j0 * pitch + (unsigned)(min(i, X + 1) + 1);
-  auto p0_of = [&](int r, double px_, double py_) -> double {
-    if (inner_col && r >= 1 && r <= Y && !(src_rows && r == g.source_row)) return px_ + py_;
-    if (!inwin) return 0.0;
-    return p0_edge(g, a.pnx, a.pny, i, r, t_prev);
-  };
-  auto rho_of = [&](double fa) -> double { return a.rho_const ? g.rho_inf : (1.0 - fa) * g.rho_inf; };
-  auto predict = [&](long k, double fa) -> double {
-    const double v = G::stored(3.0 * fa - 3.0 * a.fgB.get(k) + a.fgC.get(k));
-    a.fgC.put(k, v);
-    return v;
-  };
-  // Ring slot of field fld of chunk row rr (row j0 - 1 + rr); each lane only
-  // touches its own column.
-  auto slot = [&](int rr, int fld) -> double* { return &ring[threadIdx.y][rr % STAGES][fld][lane]; };
-  // Queue the copies of chunk row rr: pnx, pny, fgA for rows j0-1..j1+1,
-  // vy_old for j0-1..j1, vx_old, fgB, fgC for j0..j1.  One commit group per
-  // row, empty past the chunk, so that a fixed wait count always means "the
-  // next row landed".
-  auto issue = [&](int rr) {
-    const int r = j0 - 1 + rr;
-    if (rr <= ROWS + 1 && r <= j1 + 1) {
-      const unsigned k = kb + (unsigned)rr * pitch;
-      a.pnx.stage(slot(rr, 0), k);
-      a.pny.stage(slot(rr, 1), k);
-      a.fgA.stage(slot(rr, 2), k);
-      if (r <= j1) {
-        a.vy_old.stage(slot(rr, 4), k);
-        if (rr >= 1) {
-          a.vx_old.stage(slot(rr, 3), k);
-          a.fgB.stage(slot(rr, 5), k);
-          a.fgC.stage(slot(rr, 6), k);
-        }
-      }
-    }
-    __pipeline_commit();
-  };
-#pragma unroll
-  for (int rr = 0; rr < STAGES; rr++) issue(rr);
-  __pipeline_wait_prior(STAGES - 2);  // rows j0-1 and j0 have landed
-
-  // Row below the chunk and the chunk's first row.
-  double pxc, pyc, fac, p0b, rhob, vyob;
-  {
-    const double pxb = S::staged(slot(0, 0)), pyb = S::staged(slot(0, 1));
-    const double fab = G::staged(slot(0, 2));
-    vyob = V::staged(slot(0, 4));
-    pxc = S::staged(slot(1, 0));
-    pyc = S::staged(slot(1, 1));
-    fac = G::staged(slot(1, 2));
-    p0b = p0_of(j0 - 1, pxb, pyb);
-    rhob = rho_of(fab);
-    if (j0 == 1 && own) predict(f.idx(i, 0), fab);
-  }
-  issue(STAGES);  // reuses the slot of row j0-1
-  double p0c = p0_of(j0, pxc, pyc), rhoc = rho_of(fac);
-  double vyd = 0.0;
-  if (cell) {
-    double pre_d;
-    vyd = vy_face_value(g, j0 - 1, vyob, p0b, p0c, face_q(g, rhob, rhoc), xm, t_cur, pre_d);
-    if (j0 == 1) {
-      a.vy_new.put(f.idx(i, 0), vyd);
-      if (!g.pml_y0) a.vy_new.put(f.idx(i, -1), pre_d);
-    }
-  }
-
-  // Per-column coefficients: PML factors of the east face and of the cell's x
-  // component, and the cylindrical metrics.
-  const double vax_e = face ? g.vax[i + 1] : 1.0, vbx_e = face ? g.vbx[i + 1] : 1.0;
-  const double pax_c = cell ? g.pax[i] : 1.0, pbx_c = cell ? g.pbx[i] : 1.0;
-  const double xu_w = cell && g.cyl ? g.xu[i] : 0.0, xu_e = cell && g.cyl ? g.xu[i + 1] : 0.0;
-  const double rxp_c = cell && g.cyl ? g.rxp[i] : 0.0;
-  const bool zero_e = (i == 0 && !g.pml_x0) || (i == X && !g.pml_x1);
-
-  // One form of the updates serves every cell: the PML factors are exactly 1
-  // outside the PML, and the divisions of the mixture density and of the
-  // void-fraction rate run only in warps that hold void fraction (a branch
-  // taken by the whole warp or skipped by it).  Special y faces (the y0 wall or
-  // source face, the source row) are whole rows, so their branch is uniform
-  // across the warp too.
-  unsigned long long res = 0ull;  // max |dp0| as a bit pattern (NaN sorts above every number)
-#pragma unroll 1
-  for (int jj = 0; jj < ROWS; jj++) {
-    const int j = j0 + jj;
-    if (j > j1) break;
-    const unsigned k = kb + (unsigned)(jj + 1) * pitch;  // (i, j) for every lane that stores
-    __pipeline_wait_prior(STAGES - 2);              // row j+1 has landed
-    const double pxn = S::staged(slot(jj + 2, 0)), pyn = S::staged(slot(jj + 2, 1));
-    const double fan = G::staged(slot(jj + 2, 2));
-    const double vxo = V::staged(slot(jj + 1, 3)), vyo = V::staged(slot(jj + 1, 4));
-    const double fgp = G::stored(3.0 * fac - 3.0 * G::staged(slot(jj + 1, 5)) + G::staged(slot(jj + 1, 6)));
-    if (own) a.fgC.put(k, fgp);
-    const double p0n = p0_of(j + 1, pxn, pyn), rhon = rho_of(fan);
-    const double p0r = __shfl_down_sync(full, p0c, 1), rhor = __shfl_down_sync(full, rhoc, 1);
-    // dt / mean(rho) of the east and north faces and the void-fraction rate h.
-    double q_e = g.dt_rho, q_n = g.dt_rho, h = 0.0;
-    if (__any_sync(full, rhoc != g.rho_inf || rhor != g.rho_inf || rhon != g.rho_inf || fgp != 0.0 || fac != 0.0)) {
-      q_e = face_q(g, rhoc, rhor);
-      q_n = face_q(g, rhoc, rhon);
-      h = void_rate_half(g, fgp, fac);
-    }
-    double fe = velocity_face_q(g, vxo, p0c, p0r, q_e, vax_e, vbx_e);
-    if (zero_e) fe = 0.0;
-    const double fw = __shfl_up_sync(full, fe, 1);
-    double pre_u;
-    const double vyu = vy_face_value(g, j, vyo, p0c, p0n, q_n, xm, t_cur, pre_u);
-    const double s1x = g.cyl ? (-xu_w * fw + xu_e * fe) * g.rdx * rxp_c : (-fw + fe) * g.rdx;
-    const double s1y = (-vyd + vyu) * g.rdy;
-    const double qx = pressure_component(g, pxc, pax_c, pbx_c, s1x, h);
-    const double qy = pressure_component(g, pyc, g.pay[j], g.pby[j], s1y, h);
-    if (cell) {
-      a.vx_new.put(k, fe);
-      a.vy_new.put(k, vyu);
-      a.px.put(k, qx);
-      a.py.put(k, qy);
-      double p0new = qx + qy;
-      if (src_rows && j == g.source_row) p0new = source_row_pressure(g, xm, t_cur);
-      res = max(res, (unsigned long long)__double_as_longlong(fabs(p0c - p0new)));
-    } else if (lane == 0 && i == 0) {
-      a.vx_new.put(k, fe);  // the x0 face, vx(0, j)
-    }
-    vyd = vyu;
-    pxc = pxn;
-    pyc = pyn;
-    fac = fan;
-    p0c = p0n;
-    rhoc = rhon;
-    issue(jj + 1 + STAGES);  // reuses the slot of row j
-  }
-  if (j1 == Y && own) predict(f.idx(i, Y + 1), fac);
-  // Warp maximum, one atomic per warp with a nonzero residual (no block
-  // barrier: the warps of a block finish their strips at different times).
-  for (int o = 16; o > 0; o >>= 1) res = max(res, __shfl_xor_sync(0xffffffffu, res, o));
-  if (lane == 0 && res) atomicMax(a.residual, res);
-}
+constexpr long kMarchWarpsWanted = 148 * 12;  // of the 148 x 16 the GPU holds
+constexpr int kMarchRows = 8;  // default of the tuned rows (crp_set_tuning)
 
 }  // namespace crp
 #include "fdtd_tma.cuh"
+#include "fdtd_march.cuh"
 namespace crp {
 
 // Velocity ghost cells (VelocityBoundaryKernel, inc/bubble_CUDA_kernel.cuh:701-811,
@@ -1396,17 +1214,48 @@ struct Scalars {
   int pipe_err;                 // nonzero: an mbarrier wait of the FDTD pass ran out (never cleared)
 };
 
-// Fast2Sum time step (src/bubble_CUDA.cu:208-212), written by the host path.
-// Start of a host-driven step: the step's times, and the residual and the
-// bubble-motion flags cleared (one launch instead of a kernel and two memsets).
-__global__ void set_time(Scalars* s, double t_prev, double t, double carry) {
-  s->t[0] = t_prev;
-  s->t[1] = t;
-  s->t[2] = carry;
-  s->residual = 0ull;
-  s->moved = 0;
-  for (int k = 0; k < 4; k++) s->bbox[k] = 0;
-  s->loop = 0;
+// The source's row for a step from t_prev to t_cur (SourceRows): out holds three
+// rows of X + 2 values.
+__device__ __forceinline__ void source_rows_cell(const GridParams& g, int i, double t_prev, double t_cur, double* out) {
+  if (i < 1 || i > g.f.X) return;
+  const double xm = ((double)i - 0.5) * g.dx, ym = ((double)g.source_row - 0.5) * g.dy;
+  const int w = g.f.X + 2;
+  double v;
+  if (source_value(g, true, xm, ym, t_prev, v)) out[i] = v;
+  if (source_value(g, true, xm, ym, t_cur, v)) out[w + i] = v;
+  if (source_value(g, false, xm, (double)g.source_row * g.dy, t_cur, v)) out[2 * w + i] = v;
+}
+constexpr int kSourceThreads = 64;
+__global__ void __launch_bounds__(kSourceThreads) source_rows(const __grid_constant__ GridParams g, const Scalars* s,
+                                                              double* out) {
+  source_rows_cell(g, blockIdx.x * kSourceThreads + threadIdx.x, s->t[0], s->t[1], out);
+}
+// The rows of up to kSourceBatch steps, step q (blockIdx.y) from t[q] to t[q + 1].
+constexpr int kSourceBatch = 32;
+struct SourceTimes {
+  double t[kSourceBatch + 1];
+};
+__global__ void __launch_bounds__(kSourceThreads) source_rows_batch(const __grid_constant__ GridParams g,
+                                                                    const __grid_constant__ SourceTimes s,
+                                                                    double* out) {
+  const int q = blockIdx.y;
+  source_rows_cell(g, blockIdx.x * kSourceThreads + threadIdx.x, s.t[q], s.t[q + 1],
+                   out + 3 * (size_t)q * (g.f.X + 2));
+}
+// Start of a host-driven step: the step's times (Fast2Sum, src/bubble_CUDA.cu:208-212),
+// the residual and the bubble-motion flags cleared, and the source's row.
+__global__ void __launch_bounds__(kSourceThreads) step_begin(const __grid_constant__ GridParams g, Scalars* s,
+                                                             double t_prev, double t, double carry, double* out) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    s->t[0] = t_prev;
+    s->t[1] = t;
+    s->t[2] = carry;
+    s->residual = 0ull;
+    s->moved = 0;
+    for (int k = 0; k < 4; k++) s->bbox[k] = 0;
+    s->loop = 0;
+  }
+  source_rows_cell(g, blockIdx.x * kSourceThreads + threadIdx.x, t_prev, t, out);
 }
 // Start of a Picard iteration of a host-driven step: residual and work-queue
 // head cleared; `done` iterations of this step have completed.
@@ -1570,7 +1419,7 @@ __global__ void ctl_end(Scalars* s, const CtlParams c) {
   s->launches[0] += 1;
   s->launches[1] += s->loop;
   s->launches[2] += s->loop;
-  s->launches[3] += 4 + (c.nb > 0) + (s->entered ? 4 + s->loop + (s->rebuilt ? 6 : 0) : 0);
+  s->launches[3] += 5 + (c.nb > 0) + (s->entered ? 4 + s->loop + (s->rebuilt ? 6 : 0) : 0);
   s->steps++;
   s->picard_last = s->loop;
   s->picard_total += s->loop;
@@ -1605,6 +1454,7 @@ struct Sim {
   bool mixed = false;
   double* scratch = nullptr;  // dense (X+2) x (Y+2) doubles for readback
   double* d_sigma = nullptr;
+  double* src_buf = nullptr;  // the source's row of the step (SourceRows)
   double* d_elem = nullptr;  // source elements: amplitude factors, then phase offsets
   // Tensor maps of every field buffer for fdtd_tma: velocity [vx, vy][buffer],
   // split pressure [px, py][buffer], void-fraction ring.
@@ -1669,7 +1519,7 @@ struct Sim {
   int couple_graph_grid = 1;  // blocks of the graph steps' coupling launch (striding over the box's tiles)
   // Launch tuning (crp_set_tuning): rows per FDTD strip chunk and the radius
   // kernel's block count (0: rp_grid_full).
-  int strip_rows = kStripRows;
+  int strip_rows = kMarchRows;
   int rp_blocks_req = 0;
   // Graph steps queued by graphs_enqueue and not yet completed by graphs_finish.
   struct Pending {
@@ -1718,6 +1568,7 @@ struct Sim {
     scratch = carve<double>((size_t)(f.X + 2) * (f.Y + 2), off, dry);
     d_sigma = carve<double>(hs.sigma_block.size(), off, dry);
     d_elem = carve<double>(2 * (size_t)std::max(cfg.ext_elements, 1), off, dry);
+    src_buf = carve<double>(3 * (size_t)(f.X + 2) * (hs.nb > 0 ? 1 : kSourceBatch), off, dry);
     d_scalars = carve<Scalars>(1, off, dry);
     if (!dry) {
       d_residual = &d_scalars->residual;
@@ -1941,6 +1792,8 @@ struct Sim {
     gp.pml_x1 = cfg.pml_x1;
     gp.pml_y0 = cfg.pml_y0;
     gp.pml_y1 = cfg.pml_y1;
+    gp.px0 = cfg.pml_x0 ? cfg.pml_grid_number : 0;
+    gp.px1 = cfg.pml_x1 ? cfg.grid_x - cfg.pml_grid_number + 1 : cfg.grid_x + 2;
     gp.cyl = cfg.tr_cylindrical;
     gp.plane_p = cfg.tr_plane_p;
     gp.focused_p = cfg.tr_focused_p;
@@ -2095,21 +1948,24 @@ struct Sim {
     return CRP_OK;
   }
 
-  // The first part of every step: the step's times (compensated sum,
-  // src/bubble_CUDA.cu:208-212), set_time and the FDTD pass, with the buffer
-  // rotations.
-  cudaError_t queue_fdtd_step() {
-    t_prev = tstep;
-    double s1 = tstep;
-    tstep = tstep + gp.dt + tstepx;
-    double s2 = tstep - s1;
-    tstepx = gp.dt + tstepx - s2;
-    cudaError_t e = launch(kClassOther, [&] { set_time<<<1, 1, 0, stream>>>(d_scalars, t_prev, tstep, tstepx); });
-    if (e != cudaSuccess) return e;
+  int source_blocks() const {
+    return src_pressure(gp) || src_velocity(gp) ? (gp.f.X + kSourceThreads) / kSourceThreads : 1;
+  }
+
+  // The next step's times (compensated sum, src/bubble_CUDA.cu:208-212).
+  static void advance(double& t, double& carry, double& before, double dt) {
+    before = t;
+    t = t + dt + carry;
+    const double s2 = t - before;
+    carry = dt + carry - s2;
+  }
+  // The FDTD pass of a step, with the buffer rotations; src: the source's row.
+  cudaError_t queue_fdtd(const double* src) {
     const int nv = cur_v ^ 1, np = cur_p ^ 1;
     // Ring rotation of store_variables: the predicted f_g goes to the f_gm buffer.
     const int a = fg_a, b = fg_b, c = fg_c;
-    e = mixed ? launch_fdtd<PrecMixed>(nv, np, a, b, c) : launch_fdtd<PrecFP64>(nv, np, a, b, c);
+    const cudaError_t e = mixed ? launch_fdtd<PrecMixed>(nv, np, a, b, c, src)
+                                : launch_fdtd<PrecFP64>(nv, np, a, b, c, src);
     if (e != cudaSuccess) return e;
     cur_v = nv;
     cur_p = np;
@@ -2118,6 +1974,18 @@ struct Sim {
     fg_c = b;  // f_gm
     return cudaSuccess;
   }
+  // The first part of a step: its times, step_begin and the FDTD pass.
+  cudaError_t queue_fdtd_step() {
+    advance(tstep, tstepx, t_prev, gp.dt);
+    const cudaError_t e = launch(kClassOther, [&] {
+      step_begin<<<source_blocks(), kSourceThreads, 0, stream>>>(gp, d_scalars, t_prev, tstep, tstepx, src_buf);
+    });
+    return e != cudaSuccess ? e : queue_fdtd(src_buf);
+  }
+  // Velocity ghost cells: written by bubble_move with bubbles, here without.
+  cudaError_t launch_ghosts() {
+    return mixed ? launch_vghost<F32c>() : launch_vghost<F64>();
+  }
 
   // Steps of a simulation without bubbles (no temperature branch, profiling or
   // Picard trace): nothing the host decides depends on a step's scalars, so
@@ -2125,9 +1993,36 @@ struct Sim {
   // scalars once, after the last.  The FDTD pass's error flag is sticky and
   // a non-finite pressure stays non-finite in the linear bubble-free step, so
   // the last step's scalars carry what step_once would have found at any step.
+  // Nothing reads the ghost velocities or the residual of the steps before the
+  // last, and the source's rows are evaluated for up to kSourceBatch steps at
+  // once, so a step is one launch (1001 x 1531, 100 steps: 36 us a step with the
+  // three launches, 26 with one).
   bool plain_ok() const { return hs.nb == 0 && !temperature_on && !prof.on && !debug_picard && stats.steps > 0; }
-  crp_status queue_plain() {
-    CRP_CUDA(queue_fdtd_step());
+  int src_next = 0, src_n = 0;  // steps of the current batch used and evaluated
+  // One step, `left` more to follow in this call.
+  crp_status queue_plain(int left) {
+    if (fdtd_tma_on) {
+      CRP_CUDA(queue_fdtd_step());
+    } else {
+      if (src_next == src_n) {
+        SourceTimes st;
+        src_n = std::min(left + 1, kSourceBatch);
+        src_next = 0;
+        double t = tstep, carry = tstepx, before;
+        st.t[0] = t;
+        for (int q = 0; q < src_n; q++) {
+          advance(t, carry, before, gp.dt);
+          st.t[q + 1] = t;
+        }
+        const dim3 grid(source_blocks(), src_n);
+        CRP_CUDA(launch(kClassOther,
+                        [&] { source_rows_batch<<<grid, kSourceThreads, 0, stream>>>(gp, st, src_buf); }));
+      }
+      advance(tstep, tstepx, t_prev, gp.dt);
+      if (left == 0) CRP_CUDA(cudaMemsetAsync(d_residual, 0, sizeof(*d_residual), stream));
+      CRP_CUDA(queue_fdtd(src_buf + 3 * (size_t)(gp.f.X + 2) * src_next++));
+    }
+    if (left == 0) CRP_CUDA(launch_ghosts());
     // The support boxes as step_once leaves them without bubbles.
     const Box snow = box_union(supp[0], box_union(supp[1], supp[2]));
     couple_box = box_union(box_union(Box{1, 1, 0, 0}, supp[0]), box_union(supp[1], supp[2]));
@@ -2155,6 +2050,7 @@ struct Sim {
   crp_status step_once() {
     CRP_CUDA(queue_fdtd_step());
     if (hs.nb > 0) CRP_CUDA(mixed ? launch_move<PrecMixed>() : launch_move<PrecFP64>());
+    else CRP_CUDA(launch_ghosts());
     // The first radius solve is queued right behind the read-back of the
     // prediction's scalars, and picard_gate decides on the device whether it
     // runs, so that the GPU does not idle while the host decides.  Not while
@@ -2289,7 +2185,7 @@ struct Sim {
   // ---- Graph path --------------------------------------------------------
   // One mixture step as a CUDA graph whose control flow runs on the device:
   //   ctl_step_begin -> IF(step ok) {
-  //     fdtd_strip, bubble_move (with the ghost cells), ctl_enter -> IF(Picard needed) {
+  //     source_rows, fdtd_march, bubble_move (with the ghost cells), ctl_enter -> IF(Picard needed) {
   //       ctl_bins -> IF(bins stale) { counting sort } -> solve order ->
   //       WHILE(residual > threshold) { bubble_rp, couple_press, ctl_iter } }
   //     -> ctl_end }
@@ -2400,8 +2296,12 @@ struct Sim {
     const int sv = cur_v, sp = cur_p, sa = fg_a, sb = fg_b, sc = fg_c;
     cudaError_t be = capture(body1, {}, sinks, [&]() -> cudaError_t {
       const int nv = cur_v ^ 1, np = cur_p ^ 1;
-      cudaError_t x = mixed ? launch_fdtd<PrecMixed>(nv, np, fg_a, fg_b, fg_c)
-                            : launch_fdtd<PrecFP64>(nv, np, fg_a, fg_b, fg_c);
+      cudaError_t x = launch(kClassOther, [&] {
+        source_rows<<<source_blocks(), kSourceThreads, 0, stream>>>(gp, ds, src_buf);
+      });
+      if (x != cudaSuccess) return x;
+      x = mixed ? launch_fdtd<PrecMixed>(nv, np, fg_a, fg_b, fg_c, src_buf)
+                : launch_fdtd<PrecFP64>(nv, np, fg_a, fg_b, fg_c, src_buf);
       if (x != cudaSuccess) return x;
       rotate_once();
       if (hs.nb > 0) {
@@ -2559,8 +2459,9 @@ struct Sim {
     int k = 0;
     while (k < n && (stats.steps == 0 || prof.on || !graphs_on || hs.nb == 0 || debug_picard || temperature_on)) {
       if (plain_ok()) {
+        src_next = src_n = 0;
         for (; k < n; k++) {
-          const crp_status st = queue_plain();
+          const crp_status st = queue_plain(n - k - 1);
           if (st != CRP_OK) return st;
         }
         return finish_plain();
@@ -2614,9 +2515,19 @@ struct Sim {
     return fail(CRP_ERR_INVALID, "unknown field");
   }
 
+  // Rows per chunk of the FDTD pass: half the tuned number, fewer where that would
+  // leave the GPU short of warps (kMarchWarpsWanted).  Measured with 4 and 8 rows:
+  // 1001 x 1531 without bubbles 26.0 and 27.5 us, 1024 x 2048 with bubbles 40.1 and 46.6
+  // (the few chunks with void fraction, the slowest, end last).
+  int march_rows(int strips) const {
+    int rows = strip_rows / 2;
+    while (rows > 1 && (long)strips * ((gp.f.Y + rows - 1) / rows) < kMarchWarpsWanted) rows >>= 1;
+    return rows;
+  }
+
   // Per-precision launches.
   template <typename P>
-  cudaError_t launch_fdtd(int nv, int np, int a, int b, int c) {
+  cudaError_t launch_fdtd(int nv, int np, int a, int b, int c, const double* src) {
     using V = typename P::V;
     using S = typename P::S;
     using G = typename P::G;
@@ -2635,6 +2546,15 @@ struct Sim {
     fa.tdev = d_scalars->t;
     fa.rho_const = stats.steps == 0 ? 1 : 0;
     fa.residual = d_residual;
+    fa.bubbles = hs.nb > 0 ? 1 : 0;
+    for (int q = 0; q < 3; q++) {
+      fa.supp[q][0] = supp[q].i0;
+      fa.supp[q][1] = supp[q].j0;
+      fa.supp[q][2] = supp[q].i1;
+      fa.supp[q][3] = supp[q].j1;
+    }
+    fa.src = SourceRows{src, src + (gp.f.X + 2), src + 2 * (gp.f.X + 2)};
+    fa.dsupp = capturing ? &d_scalars->supp[0][0] : nullptr;
     cudaError_t e;
     if (fdtd_tma_on) {
       TmaMaps m;
@@ -2650,21 +2570,18 @@ struct Sim {
       int* perr = &d_scalars->pipe_err;
       e = launch(kClassFdtd, [&] { fdtd_tile<P><<<grid, block, smem, stream>>>(gp, fa, m, ntx, nt, perr); });
     } else {
-      const int strips = (gp.f.X + kStripCells - 1) / kStripCells, rows = strip_rows;
-      dim3 block(32, kStripWarps);
-      dim3 grid((strips + kStripWarps - 1) / kStripWarps, (gp.f.Y + rows - 1) / rows);
-      if (rows == 4)
-        e = launch(kClassFdtd, [&] { fdtd_strip<P, kStripStages, 4><<<grid, block, 0, stream>>>(gp, fa); });
-      else if (rows == 16)
-        e = launch(kClassFdtd, [&] { fdtd_strip<P, kStripStages, 16><<<grid, block, 0, stream>>>(gp, fa); });
-      else
-        e = launch(kClassFdtd, [&] { fdtd_strip<P><<<grid, block, 0, stream>>>(gp, fa); });
+      const int strips = (gp.f.X + kMarchCols - 1) / kMarchCols, rows = march_rows(strips);
+      const int chunks = (gp.f.Y + rows - 1) / rows;
+      const int grid = strips * ((chunks + kMarchWarps - 1) / kMarchWarps);
+      e = launch(kClassFdtd, [&] { fdtd_march<P><<<grid, 32 * kMarchWarps, 0, stream>>>(gp, fa, rows, strips); });
     }
-    if (e != cudaSuccess) return e;
-    if (hs.nb > 0) return cudaSuccess;  // bubble_move, which follows, writes the ghost cells
+    return e;
+  }
+  template <typename V>
+  cudaError_t launch_vghost() {
     const int ng = vghost_threads(gp.f);
-    const V vxn = view<V>(vx[nv]), vyn = view<V>(vy[nv]);
-    return launch(kClassOther, [&] { vghost<V><<<(ng + 255) / 256, 256, 0, stream>>>(gp, vxn, vyn); });
+    const V x = view<V>(vx[cur_v]), y = view<V>(vy[cur_v]);
+    return launch(kClassOther, [&] { vghost<V><<<(ng + 255) / 256, 256, 0, stream>>>(gp, x, y); });
   }
 
   // Source elements (crp_set_source_elements).
@@ -3172,9 +3089,10 @@ crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, d
   std::vector<double> times((size_t)N + 1);
   times[0] = tstep;
   bool queued = false;  // steps queued by queue_plain, checked by finish_plain
+  src_next = src_n = 0;
   for (int n = 1; n <= N; n++) {
     const bool plain = plain_ok();
-    const crp_status st = plain ? queue_plain() : step_once();
+    const crp_status st = plain ? queue_plain(N - n) : step_once();
     if (st != CRP_OK) return st;
     queued = queued || plain;
     double* out = hist + (size_t)(n - 1) * cells_box;
