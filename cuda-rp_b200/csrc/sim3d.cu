@@ -10,10 +10,8 @@
 // Kernels of one mixture step:
 //   fdtd3        fused velocity update (three faces per cell), void-fraction
 //                prediction, split-pressure update, source forcing and
-//                residual; a 32 x 8 block of threads holds a 30 x 6 patch of
-//                cells (and a ring of halo cells) and marches along z, the face
-//                below in registers, x-neighbours by shuffle, y-neighbours
-//                through shared memory: one pass over the state
+//                residual; warps of 64 columns march along z, the face below
+//                in registers: one pass over the state
 //   move3        bubble state rotation, velocity gather over the staggered
 //                2 x 2 x 2 stencils, motion, cell indices, bounding box
 //   bin3_*       counting sort of bubbles by cell (when a bubble changed cell)
@@ -59,6 +57,7 @@ struct Grid3 {
   double dx, dy, dz, rdx, rdy, rdz, dt;
   double rho_inf, c_inf, P_inf;
   double dt_rho, s3p;  // dt / rho_inf, dt rho_inf c_inf^2
+  int px0, px1;        // cells i <= px0 and i >= px1 lie in the x PML
   // PML factors 1 - s and 1 / (1 + s): faces va?/vb?[n + 1], n in [-1, N+1];
   // cells pa?/pb?[n], n in [0, N+1].
   const double *vax, *vbx, *vay, *vby, *vaz, *vbz, *pax, *pbx, *pay, *pby, *paz, *pbz;
@@ -86,15 +85,6 @@ __device__ __noinline__ double element_pressure(const Grid3& g, int e, double t)
   return g.pamp * g.elem_amp[e] * burst_env(g, tau) * sin(g.omega * t + g.elem_phase[e]);
 }
 
-__device__ __forceinline__ double face_q3(const Grid3& g, double ra, double rb) {
-  return (ra == g.rho_inf && rb == g.rho_inf) ? g.dt_rho : g.dt / ((ra + rb) * 0.5);
-}
-// (v_old (1 - s3) - dt / mean(rho) (p0b - p0a) / h) / (1 + s3), with the face's
-// PML factors fa = 1 - s3 and fb = 1 / (1 + s3).
-__device__ __forceinline__ double face3(double v_old, double p0a, double p0b, double q, double rh, double fa,
-                                        double fb) {
-  return (v_old * fa - q * ((-p0a + p0b) * rh)) * fb;
-}
 __device__ __forceinline__ double void_half3(const Grid3& g, double fg, double fgn) {
   if (fg == 0.0 && fgn == 0.0) return 0.0;
   return 0.5 * (-(fg - fgn) / g.dt / (1.0 - 0.5 * (fg + fgn)));
@@ -105,176 +95,264 @@ struct Fdtd3Args {
   typename P::V vx_old, vy_old, vz_old, vx_new, vy_new, vz_new;
   typename P::S pnx, pny, pnz, px, py, pz;
   typename P::G fgA, fgB, fgC;  // f_g, f_gn, f_gm of the previous step; fgC receives the prediction
-  const double* tdev;           // {t_prev, t_cur}
   int rho_const;
+  // Where the void fraction can be nonzero: whether there are bubbles, and the
+  // support boxes {i0, j0, k0, i1, j1, k1} of the last three steps.
+  int bubbles;
+  int supp[3][6];
+  const double* elem_p;  // pressure of every source element at the end of the step
   unsigned long long* residual;
 };
 
-constexpr int kTX = 32, kTY = 8;   // threads per block
-constexpr int kCX = 30, kCY = 6;   // cells updated per block
-constexpr int kZChunk = 32;        // planes per block
-constexpr int kStages3 = 4;        // ring slots (planes) per thread
-constexpr int kFields3 = 9;        // pnx, pny, pnz, fgA, vx_old, vy_old, vz_old, fgB, fgC
-constexpr size_t kRing3Bytes = sizeof(double) * kStages3 * kFields3 * kTX * kTY;
+// The fused pass over the grid.  A warp covers 64 columns of one row, two adjacent
+// ones per lane (16-byte accesses), and marches up a chunk of planes; a block's warps
+// take consecutive rows.  The plane below stays in registers and the next one is
+// loaded ahead; the neighbours across rows and columns are read again (the block's
+// other warps have just loaded them) and the west and south faces formed twice, so
+// that no thread waits for another: no shared memory, no barriers.
+//
+// As in the 2-D pass the void fraction takes part only where the supports of the last
+// three steps say that it can be nonzero: 96 bytes per cell elsewhere instead of
+// 128, and no divisions.
+//
+// Bound by the latency of its loads at 16 warps per SM (128 registers); DRAM traffic is
+// 1.14 times the 96 bytes per cell.  256^3 with a small cloud 366 us (4.4 TB/s of the 96
+// bytes; 718 before, with each thread's inputs staged through shared memory and two
+// barriers per plane), 141 x 125 x 133 without bubbles 70 us (155).
+constexpr int kRows3 = 8;   // warps per block
+constexpr int kCols3 = 64;  // columns per warp
+constexpr int kPlanes3 = 16;  // planes per chunk, at most
+constexpr double kCloudShare3 = 0.25;
 
-// Each thread's inputs of plane k0 - 1 + r are staged in ring slot r % kStages3
-// (dynamic shared memory, one 8-byte element per thread and field) by
-// asynchronous copies issued kStages3 - 2 planes ahead, so the loads of the
-// next planes are in flight while a plane is computed.
+enum March3Form { kPlain3 = 0, kEdges3 = 1, kVoid3 = 2 };  // inside; with x PML; with void fraction as well
+
+template <typename S>
+struct Three {
+  double2 x, y, z;
+  __device__ __forceinline__ double2 sum() const { return make_double2(x.x + y.x + z.x, x.y + y.y + z.y); }
+};
+
+// The predictions of the ghost cells beside a boundary cell (every combination of
+// the faces it touches).
 template <typename P>
-__global__ void __launch_bounds__(kTX* kTY, 2) fdtd3(const __grid_constant__ Grid3 g, const Fdtd3Args<P> a) {
+__device__ __noinline__ void predict_ghosts3(const Grid3& g, const Fdtd3Args<P>& a, int i, int j, int k) {
+  using G = typename P::G;
+  const Frame3& f = g.f;
+  const int gi = i == 1 ? 0 : (i == f.X ? f.X + 1 : -2);
+  const int gj = j == 1 ? 0 : (j == f.Y ? f.Y + 1 : -2);
+  const int gk = k == 1 ? 0 : (k == f.Z ? f.Z + 1 : -2);
+  for (int ci = 0; ci < 2; ci++)
+    for (int cj = 0; cj < 2; cj++)
+      for (int ck = 0; ck < 2; ck++) {
+        if (!(ci || cj || ck)) continue;
+        if ((ci && gi == -2) || (cj && gj == -2) || (ck && gk == -2)) continue;
+        const long q = f.idx(ci ? gi : i, cj ? gj : j, ck ? gk : k);
+        a.fgC.put(q, G::stored(3.0 * a.fgA.get(q) - 3.0 * a.fgB.get(q) + a.fgC.get(q)));
+      }
+}
+
+// Columns i and i + 1 (i odd, i <= X) of row j, planes k0..k1.
+template <typename P, int FORM>
+__device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const Fdtd3Args<P>& a, int i, int j,
+                                                           int k0, int k1) {
   using G = typename P::G;
   using S = typename P::S;
-  using V = typename P::V;
-  __shared__ double s_p0[2][kTY][kTX], s_rho[2][kTY][kTX], s_vy[2][kTY][kTX];
-  extern __shared__ __align__(16) double ring3[];  // [kStages3][kFields3][kTY * kTX]
+  constexpr bool EDGE = FORM >= kEdges3, VOID = FORM == kVoid3;
   const Frame3& f = g.f;
-  const int X = f.X, Y = f.Y, Z = f.Z;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = blockIdx.x * kCX + tx, j = blockIdx.y * kCY + ty;
-  const int k0 = 1 + blockIdx.z * kZChunk, k1 = min(Z, k0 + kZChunk - 1);
-  const bool upd = tx >= 1 && tx <= kCX && ty >= 1 && ty <= kCY && i <= X && j <= Y;
-  const int il = min(i, X + 1), jl = min(j, Y + 1);  // loads of threads past the window repeat the edge
-  const double t_cur = a.tdev[1];
-  const unsigned full = 0xffffffffu;
-  auto rho_of = [&](double fa) { return a.rho_const ? g.rho_inf : (1.0 - fa) * g.rho_inf; };
-  auto predict = [&](int ii, int jj, int kk) {
-    const long q = f.idx(ii, jj, kk);
-    const double v = G::stored(3.0 * a.fgA.get(q) - 3.0 * a.fgB.get(q) + a.fgC.get(q));
-    a.fgC.put(q, v);
-    return v;
+  const bool two = i + 1 <= f.X;
+  const unsigned pitch = (unsigned)f.pitch, plane = (unsigned)(f.Y + 4) * pitch;
+  auto own = [&](unsigned q) -> Three<S> { return {a.pnx.get2(q), a.pny.get2(q), a.pnz.get2(q)}; };
+  auto one = [&](unsigned q) -> double { return a.pnx.get(q) + a.pny.get(q) + a.pnz.get(q); };
+  auto rho_of = [&](double fa) -> double { return a.rho_const ? g.rho_inf : (1.0 - fa) * g.rho_inf; };
+  // face3 with the roundings of v_old fa - q s2: the product q s2 rounded first.
+  auto face = [&](double v, double p0a, double p0b, double q, double rh, double fa, double fb) -> double {
+    return fma(v, fa, -__dmul_rn(q, (-p0a + p0b) * rh)) * fb;
   };
-  const double vax = g.vax[il + 1], vbx = g.vbx[il + 1], vay = g.vay[jl + 1], vby = g.vby[jl + 1];
-  const double pax = g.pax[il], pbx = g.pbx[il], pay = g.pay[jl], pby = g.pby[jl];
-
-  const int tid = ty * kTX + tx;
-  auto slot = [&](int r, int fld) -> double* { return &ring3[((r % kStages3) * kFields3 + fld) * (kTX * kTY) + tid]; };
-  const long qb = f.idx(il, jl, k0 - 1), plane = (long)(Y + 4) * f.pitch;
-  // Queue the copies of plane kk = k0 - 1 + r: pnx, pny, pnz, fgA for planes
-  // k0-1..k1+1, vz_old for k0-1..k1, vx_old, vy_old, fgB, fgC for k0..k1.  One
-  // commit group per plane, empty past the chunk, so that a fixed wait count
-  // always means "the next plane landed".
-  auto issue = [&](int r) {
-    const int kk = k0 - 1 + r;
-    if (kk <= k1 + 1) {
-      const long q = qb + r * plane;
-      a.pnx.stage(slot(r, 0), q);
-      a.pny.stage(slot(r, 1), q);
-      a.pnz.stage(slot(r, 2), q);
-      a.fgA.stage(slot(r, 3), q);
-      if (kk <= k1) {
-        a.vz_old.stage(slot(r, 6), q);
-        if (r >= 1) {
-          a.vx_old.stage(slot(r, 4), q);
-          a.vy_old.stage(slot(r, 5), q);
-          a.fgB.stage(slot(r, 7), q);
-          a.fgC.stage(slot(r, 8), q);
-        }
-      }
-    }
-    __pipeline_commit();
-  };
-#pragma unroll
-  for (int r = 0; r < kStages3; r++) issue(r);
-  __pipeline_wait_prior(kStages3 - 2);  // planes k0 - 1 and k0 have landed
-
-  // The face below the first plane, vz(i, j, k0 - 1), from planes k0 - 1 and k0.
-  double p0c, rhoc, fb, pxc, pyc, pzc, fac;
+  // dt / mean(rho) as face_q3 (a quotient of equal densities rho_inf is dt_rho).
+  auto slow = [&](double ra, double rb) -> double { return VOID ? quotient(g.dt, (ra + rb) * 0.5) : g.dt_rho; };
+  unsigned q = ((unsigned)k0 * (unsigned)(f.Y + 4) + (unsigned)(j + 1)) * pitch + (unsigned)(i + 1);  // plane k0 - 1
+  const double vayn = g.vay[j + 1], vbyn = g.vby[j + 1], vays = g.vay[j], vbys = g.vby[j];
+  const double pay = g.pay[j], pby = g.pby[j];
+  Three<S> cur = own(q + plane);
+  double2 pc = cur.sum();
+  double2 fc = make_double2(0.0, 0.0);  // f_g of this plane
+  double zb[2];                         // the faces below
   {
-    const double pxb = S::staged(slot(0, 0)), pyb = S::staged(slot(0, 1)), pzb = S::staged(slot(0, 2));
-    const double fab = G::staged(slot(0, 3)), vz_old_b = V::staged(slot(0, 6));
-    pxc = S::staged(slot(1, 0));
-    pyc = S::staged(slot(1, 1));
-    pzc = S::staged(slot(1, 2));
-    fac = G::staged(slot(1, 3));
-    const double p0b = pxb + pyb + pzb, rhob = rho_of(fab);
-    p0c = pxc + pyc + pzc;
-    rhoc = rho_of(fac);
-    fb = face3(vz_old_b, p0b, p0c, face_q3(g, rhob, rhoc), g.rdz, g.vaz[k0], g.vbz[k0]);
-    if (k0 == 1 && upd) a.vz_new.put(f.idx(i, j, 0), fb);
-  }
-  issue(kStages3);  // reuses the slot of plane k0 - 1
-  int src_e = g.src[qb + plane];  // source element + 1 of plane k0
-  unsigned long long res = 0ull;
-  int buf = 0;
-#pragma unroll 1
-  for (int k = k0; k <= k1; k++) {
-    const int r = k - k0 + 1;
-    __pipeline_wait_prior(kStages3 - 2);  // plane k + 1 has landed
-    // Next plane.
-    const double pxn = S::staged(slot(r + 1, 0)), pyn = S::staged(slot(r + 1, 1)), pzn = S::staged(slot(r + 1, 2));
-    const double fan = G::staged(slot(r + 1, 3));
-    const double p0n = pxn + pyn + pzn, rhon = rho_of(fan);
-    // This plane's old faces and void-fraction history.
-    const double vxo = V::staged(slot(r, 4)), vyo = V::staged(slot(r, 5)), vzo = V::staged(slot(r, 6));
-    const double fgB = G::staged(slot(r, 7)), fgC = G::staged(slot(r, 8));
-    issue(r + kStages3);  // reuses the slot of plane k
-    const int e = src_e;
-    if (k < k1) src_e = g.src[qb + (long)(r + 1) * plane];
-    s_p0[buf][ty][tx] = p0c;
-    s_rho[buf][ty][tx] = rhoc;
-    __syncthreads();
-    const double p0r = __shfl_down_sync(full, p0c, 1), rhor = __shfl_down_sync(full, rhoc, 1);
-    const double p0u = s_p0[buf][min(ty + 1, kTY - 1)][tx], rhou = s_rho[buf][min(ty + 1, kTY - 1)][tx];
-    const double fe = face3(vxo, p0c, p0r, face_q3(g, rhoc, rhor), g.rdx, vax, vbx);
-    const double fn = face3(vyo, p0c, p0u, face_q3(g, rhoc, rhou), g.rdy, vay, vby);
-    const double ft = face3(vzo, p0c, p0n, face_q3(g, rhoc, rhon), g.rdz, g.vaz[k + 1], g.vbz[k + 1]);
-    s_vy[buf][ty][tx] = fn;
-    __syncthreads();
-    const double fw = __shfl_up_sync(full, fe, 1);
-    const double fs = s_vy[buf][max(ty - 1, 0)][tx];
-    if (upd) {
-      const long o = f.idx(i, j, k);
-      a.vx_new.put(o, fe);
-      a.vy_new.put(o, fn);
-      a.vz_new.put(o, ft);
-      const double fgp = G::stored(3.0 * fac - 3.0 * fgB + fgC);
-      a.fgC.put(o, fgp);
-      // Ghost cells next to the domain's faces take their prediction from
-      // the cell beside them (every combination of the faces it touches).
-      const int gi = i == 1 ? 0 : (i == X ? X + 1 : -2);
-      const int gj = j == 1 ? 0 : (j == Y ? Y + 1 : -2);
-      const int gk = k == 1 ? 0 : (k == Z ? Z + 1 : -2);
-      if (gi > -2 || gj > -2 || gk > -2) {
-        for (int ci = 0; ci < 2; ci++)
-          for (int cj = 0; cj < 2; cj++)
-            for (int ck = 0; ck < 2; ck++) {
-              if (!(ci || cj || ck)) continue;
-              if ((ci && gi == -2) || (cj && gj == -2) || (ck && gk == -2)) continue;
-              predict(ci ? gi : i, cj ? gj : j, ck ? gk : k);
-            }
-      }
-      const double h = void_half3(g, fgp, fac);
-      const double qx = pxc * pax - g.s3p * ((-fw + fe) * g.rdx + h) * pbx;
-      const double qy = pyc * pay - g.s3p * ((-fs + fn) * g.rdy + h) * pby;
-      const double qz = pzc * g.paz[k] - g.s3p * ((-fb + ft) * g.rdz + h) * g.pbz[k];
-      double p0new = qx + qy + qz;
-      if (e > 0) {
-        p0new = element_pressure(g, e - 1, t_cur);
-        a.px.put(o, p0new);
-        a.py.put(o, 0.0);
-        a.pz.put(o, 0.0);
-      } else {
-        a.px.put(o, qx);
-        a.py.put(o, qy);
-        a.pz.put(o, qz);
-      }
-      res = max(res, (unsigned long long)__double_as_longlong(fabs(p0c - p0new)));
+    const double2 pb = own(q).sum(), vb = a.vz_old.get2(q);
+    double rb[2] = {0.0, 0.0}, rc[2] = {0.0, 0.0};
+    if (VOID) {
+      const double2 fb = a.fgA.get2(q);
+      fc = a.fgA.get2(q + plane);
+      rb[0] = rho_of(fb.x), rb[1] = rho_of(fb.y);
+      rc[0] = rho_of(fc.x), rc[1] = rho_of(fc.y);
     }
-    // The x0 and y0 faces of the domain belong to the threads on the ghost cells.
-    if (i == 0 && ty >= 1 && ty <= kCY && j <= Y) a.vx_new.put(f.idx(0, j, k), fe);
-    if (j == 0 && tx >= 1 && tx <= kCX && i <= X) a.vy_new.put(f.idx(i, 0, k), fn);
-    fb = ft;
-    pxc = pxn;
-    pyc = pyn;
-    pzc = pzn;
-    fac = fan;
-    p0c = p0n;
-    rhoc = rhon;
-    buf ^= 1;
+    zb[0] = face(vb.x, pb.x, pc.x, slow(rb[0], rc[0]), g.rdz, g.vaz[k0], g.vbz[k0]);
+    zb[1] = face(vb.y, pb.y, pc.y, slow(rb[1], rc[1]), g.rdz, g.vaz[k0], g.vbz[k0]);
+    if (k0 == 1) {
+      a.vz_new.put(q, zb[0]);
+      if (two) a.vz_new.put(q + 1, zb[1]);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) res = max(res, __shfl_xor_sync(full, res, o));
-  if (tx == 0 && res) atomicMax(a.residual, res);
+  q += plane;  // plane k0
+  Three<S> nxt = own(q + plane);
+  double2 vx2 = a.vx_old.get2(q), vy2 = a.vy_old.get2(q), vs2 = a.vy_old.get2(q - pitch), vz2 = a.vz_old.get2(q);
+  double vxl = a.vx_old.get(q - 1);
+  unsigned long long res = 0ull;
+#pragma unroll 1
+  for (int k = k0; k <= k1; k++, q += plane) {
+    const double2 vxo = vx2, vyo = vy2, vso = vs2, vzo = vz2;
+    const double vxw = vxl;
+    const Three<S> up = nxt;
+    const double2 pu = up.sum();
+    // The neighbours of this plane, then what the next one needs.
+    const double pl = one(q - 1), pr = one(q + 2);
+    const double2 ps = own(q - pitch).sum(), pn = own(q + pitch).sum();
+    const short2 e = *reinterpret_cast<const short2*>(g.src + q);
+    if (k < k1) {
+      nxt = own(q + 2 * plane);
+      vx2 = a.vx_old.get2(q + plane);
+      vy2 = a.vy_old.get2(q + plane);
+      vs2 = a.vy_old.get2(q + plane - pitch);
+      vz2 = a.vz_old.get2(q + plane);
+      vxl = a.vx_old.get(q + plane - 1);
+    }
+    double qx[3] = {g.dt_rho, g.dt_rho, g.dt_rho}, qn[2] = {g.dt_rho, g.dt_rho}, qs[2] = {g.dt_rho, g.dt_rho},
+           qz[2] = {g.dt_rho, g.dt_rho}, h[2] = {0.0, 0.0};
+    double2 fu = fc;
+    if (VOID) {
+      fu = a.fgA.get2(q + plane);
+      const double2 fs = a.fgA.get2(q - pitch), fn = a.fgA.get2(q + pitch), fB = a.fgB.get2(q), fC = a.fgC.get2(q);
+      const double fl = a.fgA.get(q - 1), fr = a.fgA.get(q + 2);
+      const double fg[2] = {G::stored(3.0 * fc.x - 3.0 * fB.x + fC.x), G::stored(3.0 * fc.y - 3.0 * fB.y + fC.y)};
+      // Nothing to divide where all of the warp's void fraction is zero, nor to store
+      // where the prediction is the stored zero.
+      const bool some = fc.x != 0.0 || fc.y != 0.0 || fu.x != 0.0 || fu.y != 0.0 || fs.x != 0.0 || fs.y != 0.0 ||
+                        fn.x != 0.0 || fn.y != 0.0 || fl != 0.0 || fr != 0.0 || fg[0] != 0.0 || fg[1] != 0.0;
+      if (some || fC.x != 0.0 || fC.y != 0.0) {
+        if (two)
+          a.fgC.put2(q, fg[0], fg[1]);
+        else
+          a.fgC.put(q, fg[0]);
+      }
+      if (i == 1 || i + 1 >= f.X || j == 1 || j == f.Y || k == 1 || k == f.Z) {
+        predict_ghosts3<P>(g, a, i, j, k);
+        if (two) predict_ghosts3<P>(g, a, i + 1, j, k);
+      }
+      if (some) {
+        const double r0 = rho_of(fc.x), r1 = rho_of(fc.y);
+        qx[0] = slow(rho_of(fl), r0);
+        qx[1] = slow(r0, r1);
+        qx[2] = slow(r1, rho_of(fr));
+        qs[0] = slow(rho_of(fs.x), r0);
+        qs[1] = slow(rho_of(fs.y), r1);
+        qn[0] = slow(r0, rho_of(fn.x));
+        qn[1] = slow(r1, rho_of(fn.y));
+        qz[0] = slow(r0, rho_of(fu.x));
+        qz[1] = slow(r1, rho_of(fu.y));
+        const double fo[2] = {fc.x, fc.y};
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+          h[c] = 0.5 * quotient(quotient(-(fg[c] - fo[c]), g.dt), 1.0 - 0.5 * (fg[c] + fo[c]));
+      }
+    }
+    const double p4[4] = {pl, pc.x, pc.y, pr}, vo[3] = {vxw, vxo.x, vxo.y};
+    double fx[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      fx[c] = face(vo[c], p4[c], p4[c + 1], qx[c], g.rdx, EDGE ? g.vax[i + c] : 1.0, EDGE ? g.vbx[i + c] : 1.0);
+    const double vaz = g.vaz[k + 1], vbz = g.vbz[k + 1], paz = g.paz[k], pbz = g.pbz[k];
+    const double yn[2] = {face(vyo.x, pc.x, pn.x, qn[0], g.rdy, vayn, vbyn),
+                          face(vyo.y, pc.y, pn.y, qn[1], g.rdy, vayn, vbyn)};
+    const double ys[2] = {face(vso.x, ps.x, pc.x, qs[0], g.rdy, vays, vbys),
+                          face(vso.y, ps.y, pc.y, qs[1], g.rdy, vays, vbys)};
+    const double zt[2] = {face(vzo.x, pc.x, pu.x, qz[0], g.rdz, vaz, vbz),
+                          face(vzo.y, pc.y, pu.y, qz[1], g.rdz, vaz, vbz)};
+    double nx[2], ny[2], nz[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      const double px = c ? cur.x.y : cur.x.x, py = c ? cur.y.y : cur.y.x, pz = c ? cur.z.y : cur.z.x;
+      // pn pa - s3p (divergence + h) pb, the last product rounded first.
+      nx[c] = fma(px, EDGE ? g.pax[i + c] : 1.0,
+                  -__dmul_rn(__dmul_rn(g.s3p, fma(-fx[c] + fx[c + 1], g.rdx, h[c])), EDGE ? g.pbx[i + c] : 1.0));
+      ny[c] = fma(py, pay, -__dmul_rn(__dmul_rn(g.s3p, fma(-ys[c] + yn[c], g.rdy, h[c])), pby));
+      nz[c] = fma(pz, paz, -__dmul_rn(__dmul_rn(g.s3p, fma(-zb[c] + zt[c], g.rdz, h[c])), pbz));
+      double p0new = nx[c] + ny[c] + nz[c];
+      const int el = c ? e.y : e.x;
+      if (el > 0) {
+        p0new = a.elem_p[el - 1];
+        nx[c] = p0new;
+        ny[c] = nz[c] = 0.0;
+      }
+      if (c == 0 || two) res = max(res, (unsigned long long)__double_as_longlong(fabs((c ? pc.y : pc.x) - p0new)));
+    }
+    if (two) {
+      a.vx_new.put2(q, fx[1], fx[2]);
+      a.vy_new.put2(q, yn[0], yn[1]);
+      a.vz_new.put2(q, zt[0], zt[1]);
+      a.px.put2(q, nx[0], nx[1]);
+      a.py.put2(q, ny[0], ny[1]);
+      a.pz.put2(q, nz[0], nz[1]);
+    } else {
+      a.vx_new.put(q, fx[1]);
+      a.vy_new.put(q, yn[0]);
+      a.vz_new.put(q, zt[0]);
+      a.px.put(q, nx[0]);
+      a.py.put(q, ny[0]);
+      a.pz.put(q, nz[0]);
+    }
+    if (i == 1) a.vx_new.put(q - 1, fx[0]);  // the x0 and y0 faces of the domain
+    if (j == 1) {
+      a.vy_new.put(q - pitch, ys[0]);
+      if (two) a.vy_new.put(q - pitch + 1, ys[1]);
+    }
+    zb[0] = zt[0];
+    zb[1] = zt[1];
+    cur = up;
+    pc = pu;
+    fc = fu;
+  }
+  return res;
+}
+
+template <typename P>
+__device__ __noinline__ unsigned long long march3_void(const Grid3& g, const Fdtd3Args<P>& a, int i, int j, int k0,
+                                                       int k1) {
+  return march3_chunk<P, kVoid3>(g, a, i, j, k0, k1);
+}
+
+// CLOUD: the supports cover much of the grid (kCloudShare3).  The void-fraction form
+// then stands in line; elsewhere it is called, so that its registers are not spilled
+// in the other forms' loops (256^3 with a small cloud 398 us in line, 366 called;
+// 384^3 with a cloud over half of the grid 1675 and 1975).
+template <typename P, bool CLOUD>
+__global__ void __launch_bounds__(32 * kRows3, 2) fdtd3(const __grid_constant__ Grid3 g,
+                                                        const __grid_constant__ Fdtd3Args<P> a, int planes) {
+  const Frame3& f = g.f;
+  const int lane = threadIdx.x, i0 = 1 + blockIdx.x * kCols3, i = i0 + 2 * lane;
+  const int j = 1 + blockIdx.y * kRows3 + threadIdx.y;
+  const int k0 = 1 + blockIdx.z * planes, k1 = min(f.Z, k0 + planes - 1);
+  if (j > f.Y) return;
+  const int i1 = min(f.X, i0 + kCols3 - 1);
+  bool fg = false;
+  if (a.bubbles) {
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      const int* b = a.supp[s];
+      fg = fg || (b[0] <= b[3] && b[1] <= b[4] && b[2] <= b[5] && b[0] <= i1 + 1 && b[3] >= i0 - 1 &&
+                  b[1] <= j + 1 && b[4] >= j - 1 && b[2] <= k1 + 1 && b[5] >= k0 - 1);
+    }
+  }
+  unsigned long long res = 0ull;
+  if (i <= f.X) {
+    if (fg)
+      res = CLOUD ? march3_chunk<P, kVoid3>(g, a, i, j, k0, k1) : march3_void<P>(g, a, i, j, k0, k1);
+    else if (i0 <= g.px0 || i1 >= g.px1)
+      res = march3_chunk<P, kEdges3>(g, a, i, j, k0, k1);
+    else
+      res = march3_chunk<P, kPlain3>(g, a, i, j, k0, k1);
+  }
+  for (int o = 16; o > 0; o >>= 1) res = max(res, __shfl_xor_sync(0xffffffffu, res, o));
+  if (lane == 0 && res) atomicMax(a.residual, res);
 }
 
 // ---------------------------------------------------------------------------
@@ -298,13 +376,32 @@ struct Scalars3 {
   unsigned long long reused;  // radius solves kept (ext.rp_reuse), summed over the handle's life
 };
 
-__global__ void set_time3(Scalars3* s, double t_prev, double t) {
+// Start of a step: its times, the accumulators cleared, and the pressure of every
+// source element at its end.
+constexpr int kBeginThreads3 = 64;
+__global__ void __launch_bounds__(kBeginThreads3) step_begin3(const __grid_constant__ Grid3 g, Scalars3* s,
+                                                              double t_prev, double t, int elems, double* elem_p) {
+  const int e = blockIdx.x * kBeginThreads3 + threadIdx.x;
+  if (e < elems) elem_p[e] = element_pressure(g, e, t);
+  if (e != 0) return;
   s->t[0] = t_prev;
   s->t[1] = t;
   s->residual = 0ull;
   s->moved = 0;
   s->box[0] = s->box[1] = s->box[2] = INT_MAX;
   s->box[3] = s->box[4] = s->box[5] = INT_MIN;
+}
+
+// Element pressures at the ends of up to kElemBatch steps (step blockIdx.y at t[q]).
+constexpr int kElemBatch = 32;
+struct ElemTimes {
+  double t[kElemBatch];
+};
+__global__ void __launch_bounds__(kBeginThreads3) elem_batch(const __grid_constant__ Grid3 g,
+                                                             const __grid_constant__ ElemTimes s, int elems,
+                                                             double* elem_p) {
+  const int e = blockIdx.x * kBeginThreads3 + threadIdx.x;
+  if (e < elems) elem_p[(size_t)blockIdx.y * elems + e] = element_pressure(g, e, s.t[blockIdx.y]);
 }
 
 __device__ __forceinline__ int bin3_of(const Frame3& f, int ix, int iy, int iz) {
@@ -660,7 +757,7 @@ struct Couple3Args {
   int box[6];  // cells [box0, box3] x [box1, box4] x [box2, box5]
   int gather;  // 1: void fraction from the bins; 0: keep fg
   int pressure;
-  const double* tdev;
+  const double* elem_p;
   unsigned long long* residual;
 };
 
@@ -703,7 +800,6 @@ __global__ void __launch_bounds__(256) couple3(const __grid_constant__ Grid3 g, 
       fgv = a.fg.get(o);
     }
     if (!same && a.pressure && i >= 1 && i <= f.X && j >= 1 && j <= f.Y && k >= 1 && k <= f.Z) {
-      const double t_cur = a.tdev[1];
       const double h = void_half3(g, fgv, a.fgn.get(o));
       const long ox = o - 1, oy = o - f.pitch, oz = o - (long)(f.Y + 4) * f.pitch;
       const double s1x = (-a.vx.get(ox) + a.vx.get(o)) * g.rdx;
@@ -716,7 +812,7 @@ __global__ void __launch_bounds__(256) couple3(const __grid_constant__ Grid3 g, 
       double p0new = qx + qy + qz;
       const int e = g.src[o];
       if (e > 0) {
-        p0new = element_pressure(g, e - 1, t_cur);
+        p0new = a.elem_p[e - 1];
         a.px.put(o, p0new);
         a.py.put(o, 0.0);
         a.pz.put(o, 0.0);
@@ -954,6 +1050,7 @@ struct Sim3Impl {
   double* d_fac = nullptr;  // PML factors
   short* d_src = nullptr;
   double* d_elem = nullptr;
+  double* elem_p = nullptr;  // pressure of every element at the end of the step
   double* scratch = nullptr;  // dense read-back
   d3::Bub3 bub{};
   int* bin_count = nullptr;
@@ -981,7 +1078,6 @@ struct Sim3Impl {
   int64_t launches = 0;
   // Profiling (crp_set_profiling): events around the FDTD launch of a step.
   bool prof_on = false, prof_pending = false;
-  bool fdtd_smem_set[2] = {false, false};  // fdtd3's dynamic shared memory limit raised (FP64, mixed)
   cudaEvent_t ev_f0 = nullptr, ev_f1 = nullptr;
   crp_status set_profiling(bool on) {
     if (on && !ev_f0) {
@@ -1026,6 +1122,7 @@ struct Sim3Impl {
     const int FX = g.f.X, FY = g.f.Y, FZ = g.f.Z;
     d_fac = carve<double>(4 * (size_t)(FX + 3 + FY + 3 + FZ + 3), off, dry);
     d_elem = carve<double>(2 * (size_t)std::max(elem_n, 1), off, dry);
+    elem_p = carve<double>((size_t)std::max(elem_n, 1) * (n > 0 ? 1 : d3::kElemBatch), off, dry);
     scratch = carve<double>((size_t)(FX + 3) * (FY + 3) * (FZ + 3), off, dry);
     d_sc = carve<d3::Scalars3>(1, off, dry);
     bub.n = n;
@@ -1056,8 +1153,23 @@ struct Sim3Impl {
 
   crp_status create(const crp_config& c, const crp_bubbles_in* bin, void* user_stream);
   crp_status step_once();
+  // Steps without bubbles, queued back to back: `left` more follow in this call.
+  // Nothing the host decides depends on their scalars; finish_plain reads those of the
+  // last step (a non-finite pressure stays non-finite in the linear step).
+  bool plain_ok() const { return bub.n == 0 && !prof_on && stats.steps > 0; }
+  int elem_next = 0, elem_made = 0;  // steps of the current batch of element pressures used and evaluated
+  crp_status queue_plain(int left);
+  crp_status finish_plain();
+  void rotate() {
+    cur_v ^= 1;
+    cur_p ^= 1;
+    const int a = fg_a, b = fg_b, c = fg_c;
+    fg_a = c;  // predicted f_g
+    fg_b = a;
+    fg_c = b;
+  }
   template <typename P>
-  crp_status launch_fdtd();
+  crp_status launch_fdtd(const double* elem);
   template <typename P>
   crp_status launch_move();
   template <typename P>
@@ -1066,6 +1178,11 @@ struct Sim3Impl {
   crp_status launch_couple(bool gather, bool pressure, const int box[6]);
   crp_status build_bins();
   crp_status build_order();
+  cudaError_t begin_step(double t0, double t1) {
+    d3::step_begin3<<<std::max(1, (elem_n + d3::kBeginThreads3 - 1) / d3::kBeginThreads3), d3::kBeginThreads3, 0,
+                      stream>>>(g, d_sc, t0, t1, elem_n, elem_p);
+    return cudaGetLastError();
+  }
   void bubble_box(int box[6]) const;
   static double as_double(unsigned long long b) {
     double d;
@@ -1180,6 +1297,8 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
   g.dt = c.sim_cfl * std::min(g.dx, std::min(g.dy, g.dz)) / g.c_inf;
   g.dt_rho = g.dt / g.rho_inf;
   g.s3p = g.dt * g.rho_inf * g.c_inf * g.c_inf;
+  g.px0 = c.pml_grid_number;
+  g.px1 = X - c.pml_grid_number + 1;
   g.omega = 2.0 * pi * c.tr_freq;
   g.pamp = g.rho_inf * g.c_inf * c.tr_amp;
   g.period = (double)(c.tr_on_wave + c.tr_off_wave) / c.tr_freq;
@@ -1332,7 +1451,7 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
     for (double* d : {bub.PG_p, bub.PG_n}) C3(up(d, pg0));
     for (double* d : {bub.dt, bub.dt_n}) C3(up(d, dt0));
     C3(cudaStreamSynchronize(stream));
-    d3::set_time3<<<1, 1, 0, stream>>>(d_sc, 0.0, 0.0);
+    C3(begin_step(0.0, 0.0));
     d3::index3_kernel<<<(nb + 255) / 256, 256, 0, stream>>>(g, bub, d_sc);
     C3(cudaGetLastError());
     {
@@ -1416,7 +1535,7 @@ crp_status Sim3Impl::build_bins() {
 }
 
 template <typename P>
-crp_status Sim3Impl::launch_fdtd() {
+crp_status Sim3Impl::launch_fdtd(const double* elem) {
   using V = typename P::V;
   using S = typename P::S;
   using G = typename P::G;
@@ -1437,18 +1556,27 @@ crp_status Sim3Impl::launch_fdtd() {
   a.fgA = view<G>(fg[fg_a]);
   a.fgB = view<G>(fg[fg_b]);
   a.fgC = view<G>(fg[fg_c]);
-  a.tdev = d_sc->t;
   a.rho_const = stats.steps == 0 ? 1 : 0;
   a.residual = &d_sc->residual;
-  const dim3 block(d3::kTX, d3::kTY);
-  const dim3 grid((g.f.X + 1 + d3::kCX - 1) / d3::kCX + 1, (g.f.Y + 1 + d3::kCY - 1) / d3::kCY + 1,
-                  (g.f.Z + d3::kZChunk - 1) / d3::kZChunk);
-  if (!fdtd_smem_set[P::kIndex]) {
-    C3(cudaFuncSetAttribute(d3::fdtd3<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d3::kRing3Bytes));
-    fdtd_smem_set[P::kIndex] = true;
-  }
+  a.bubbles = bub.n > 0 ? 1 : 0;
+  std::memcpy(a.supp, supp, sizeof(a.supp));
+  a.elem_p = elem;
+  const int sx = (g.f.X + d3::kCols3 - 1) / d3::kCols3, sy = (g.f.Y + d3::kRows3 - 1) / d3::kRows3;
+  // Planes per chunk: up to 16 (256^3: 398 us, 425 with 32, 402 with 8), fewer where that
+  // would leave less than two waves of the 296 blocks that the GPU holds.
+  int planes = d3::kPlanes3;
+  while (planes > 2 && (long)sx * sy * ((g.f.Z + planes - 1) / planes) < 4 * 148) planes /= 2;
+  const dim3 block(32, d3::kRows3), grid(sx, sy, (g.f.Z + planes - 1) / planes);
+  int u[6], w[6];
+  box_union(w, supp[0], supp[1]);
+  box_union(u, w, supp[2]);
+  const bool cloud = u[0] <= u[3] && (double)(u[3] - u[0] + 1) * (u[4] - u[1] + 1) * (u[5] - u[2] + 1) >
+                                         d3::kCloudShare3 * g.f.X * g.f.Y * g.f.Z;
   if (prof_on) C3(cudaEventRecord(ev_f0, stream));
-  d3::fdtd3<P><<<grid, block, d3::kRing3Bytes, stream>>>(g, a);
+  if (cloud)
+    d3::fdtd3<P, true><<<grid, block, 0, stream>>>(g, a, planes);
+  else
+    d3::fdtd3<P, false><<<grid, block, 0, stream>>>(g, a, planes);
   C3(cudaGetLastError());
   if (prof_on) {
     C3(cudaEventRecord(ev_f1, stream));
@@ -1521,7 +1649,7 @@ crp_status Sim3Impl::launch_couple(bool gather, bool pressure, const int box[6])
   for (int q = 0; q < 6; q++) a.box[q] = box[q];
   a.gather = gather ? 1 : 0;
   a.pressure = pressure ? 1 : 0;
-  a.tdev = d_sc->t;
+  a.elem_p = elem_p;
   a.residual = &d_sc->residual;
   const dim3 block(32, 8);
   const dim3 grid((box[3] - box[0] + 32) / 32, (box[4] - box[1] + 8) / 8, box[5] - box[2] + 1);
@@ -1531,25 +1659,65 @@ crp_status Sim3Impl::launch_couple(bool gather, bool pressure, const int box[6])
   return CRP_OK;
 }
 
+crp_status Sim3Impl::queue_plain(int left) {
+  auto advance = [&](double& t, double& carry) {
+    const double s1 = t;
+    t = t + g.dt + carry;
+    const double s2 = t - s1;
+    carry = g.dt + carry - s2;
+  };
+  if (elem_next == elem_made) {
+    d3::ElemTimes et;
+    elem_made = std::min(left + 1, d3::kElemBatch);
+    elem_next = 0;
+    double t = tstep, carry = tstepx;
+    for (int q = 0; q < elem_made; q++) {
+      advance(t, carry);
+      et.t[q] = t;
+    }
+    if (elem_n > 0) {
+      const dim3 grid((elem_n + d3::kBeginThreads3 - 1) / d3::kBeginThreads3, elem_made);
+      d3::elem_batch<<<grid, d3::kBeginThreads3, 0, stream>>>(g, et, elem_n, elem_p);
+      C3(cudaGetLastError());
+      launches++;
+    }
+  }
+  t_prev = tstep;
+  advance(tstep, tstepx);
+  if (left == 0) C3(cudaMemsetAsync(&d_sc->residual, 0, sizeof(unsigned long long), stream));
+  const double* ep = elem_p + (size_t)elem_n * elem_next++;
+  const crp_status st = mixed ? launch_fdtd<d3::PMix>(ep) : launch_fdtd<d3::P64>(ep);
+  if (st != CRP_OK) return st;
+  rotate();
+  stats.steps++;
+  stats.time = tstep;
+  stats.picard_last = 0;
+  return CRP_OK;
+}
+
+crp_status Sim3Impl::finish_plain() {
+  C3(cudaMemcpyAsync(h_sc, d_sc, sizeof(d3::Scalars3), cudaMemcpyDeviceToHost, stream));
+  C3(cudaStreamSynchronize(stream));
+  const double res = as_double(h_sc->residual) / g.P_inf;
+  if (std::isnan(res)) return fail(CRP_ERR_NONFINITE, "non-finite pressure");
+  stats.residual_last = res;
+  stats.rp_substeps_max = h_sc->substep_max;
+  stats.rp_reused = (int64_t)h_sc->reused;
+  stats.kernel_launches = launches;
+  return CRP_OK;
+}
+
 crp_status Sim3Impl::step_once() {
   t_prev = tstep;
   const double s1 = tstep;
   tstep = tstep + g.dt + tstepx;
   const double s2 = tstep - s1;
   tstepx = g.dt + tstepx - s2;
-  d3::set_time3<<<1, 1, 0, stream>>>(d_sc, t_prev, tstep);
-  C3(cudaGetLastError());
+  C3(begin_step(t_prev, tstep));
   launches++;
-  crp_status st = mixed ? launch_fdtd<d3::PMix>() : launch_fdtd<d3::P64>();
+  crp_status st = mixed ? launch_fdtd<d3::PMix>(elem_p) : launch_fdtd<d3::P64>(elem_p);
   if (st != CRP_OK) return st;
-  cur_v ^= 1;
-  cur_p ^= 1;
-  {
-    const int a = fg_a, b = fg_b, c = fg_c;
-    fg_a = c;  // predicted f_g
-    fg_b = a;
-    fg_c = b;
-  }
+  rotate();
   if (bub.n > 0) {
     st = mixed ? launch_move<d3::PMix>() : launch_move<d3::P64>();
     if (st != CRP_OK) return st;
@@ -1721,8 +1889,11 @@ crp_status Sim3Impl::adjoint(const crp_objective* obj, double* J, double* grad_a
   // Forward, recording the focal p0 after every step.
   std::vector<double> times((size_t)N + 1);
   times[0] = tstep;
+  elem_next = elem_made = 0;
   for (int n = 1; n <= N; n++) {
-    const crp_status st = step_once();
+    const bool plain = plain_ok();
+    crp_status st = plain ? queue_plain(N - n) : step_once();
+    if (plain && st == CRP_OK && n == N) st = finish_plain();
     if (st != CRP_OK) return st;
     double* out = hist + (size_t)(n - 1) * box_n;
     if (mixed)
@@ -1882,9 +2053,12 @@ crp_status sim3_create(const crp_config* cfg, const crp_bubbles_in* bubbles, voi
 }
 void sim3_destroy(Sim3Impl* s) { delete s; }
 crp_status sim3_step(Sim3Impl* s, int n) {
+  s->elem_next = s->elem_made = 0;
   for (int k = 0; k < n; k++) {
-    const crp_status st = s->step_once();
+    const bool plain = s->plain_ok();
+    const crp_status st = plain ? s->queue_plain(n - k - 1) : s->step_once();
     if (st != CRP_OK) return st;
+    if (plain && k == n - 1) return s->finish_plain();
   }
   return CRP_OK;
 }
