@@ -90,6 +90,20 @@ __device__ __forceinline__ double void_half3(const Grid3& g, double fg, double f
   return 0.5 * (-(fg - fgn) / g.dt / (1.0 - 0.5 * (fg + fgn)));
 }
 
+// Tiles of 32 x 8 x 8 cells (ghost cells included) and the last coupling in which
+// bubbles touched each (mark_tiles).  Couplings are counted by the steps whose Picard
+// loop ran.  A step's void fraction is nonzero at most where bubbles touched it in that
+// coupling, or, without one, where it was in the three steps before; so the f_g of a
+// step and of the two before it reach back six couplings at most, and a tile not
+// touched since holds zeros only.
+constexpr int kTile3X = 32, kTile3Y = 8, kTile3Z = 8, kTileLife = 6;
+struct Tiles3 {
+  int nx, ny, nz;
+  int* last;  // coupling index of the last touch (very negative: never)
+  int* list;  // active tiles of the step
+  __host__ __device__ __forceinline__ int at(int x, int y, int z) const { return (z * ny + y) * nx + x; }
+};
+
 template <typename P>
 struct Fdtd3Args {
   typename P::V vx_old, vy_old, vz_old, vx_new, vy_new, vz_new;
@@ -100,6 +114,8 @@ struct Fdtd3Args {
   // support boxes {i0, j0, k0, i1, j1, k1} of the last three steps.
   int bubbles;
   int supp[3][6];
+  Tiles3 tiles;
+  int coupling;          // index of the next coupling
   const double* elem_p;  // pressure of every source element at the end of the step
   unsigned long long* residual;
 };
@@ -341,6 +357,16 @@ __global__ void __launch_bounds__(32 * kRows3, 2) fdtd3(const __grid_constant__ 
       fg = fg || (b[0] <= b[3] && b[1] <= b[4] && b[2] <= b[5] && b[0] <= i1 + 1 && b[3] >= i0 - 1 &&
                   b[1] <= j + 1 && b[4] >= j - 1 && b[2] <= k1 + 1 && b[5] >= k0 - 1);
     }
+    if (fg) {  // the supports' boxes meet the chunk: so does an active tile?
+      const int x0 = (i0 - 1) / kTile3X, y0 = (j - 1) / kTile3Y, z0 = (k0 - 1) / kTile3Z;
+      const int nx = (i1 + 1) / kTile3X - x0 + 1, ny = (j + 1) / kTile3Y - y0 + 1, nz = (k1 + 1) / kTile3Z - z0 + 1;
+      bool live = false;
+      for (int t = lane; t < nx * ny * nz; t += 32) {
+        const int last = a.tiles.last[a.tiles.at(x0 + t % nx, y0 + t / nx % ny, z0 + t / (nx * ny))];
+        live = live || a.coupling - last <= kTileLife;
+      }
+      fg = __any_sync(0xffffffffu, live);
+    }
   }
   unsigned long long res = 0ull;
   if (i <= f.X) {
@@ -372,6 +398,7 @@ struct Scalars3 {
   int next;
   int moved;
   int box[6];  // bubbles' ibn box: min x, y, z, max x, y, z
+  int tiles;   // active tiles of this step (mark_tiles)
   double t[2];
   unsigned long long reused;  // radius solves kept (ext.rp_reuse), summed over the handle's life
 };
@@ -466,10 +493,8 @@ __device__ __forceinline__ double gather_v(const Grid3& g, const BubbleParams& b
 // (BubbleInterpolationVelocityKernel, :398-448, with its z component), the
 // motion (BubbleMotionKernel, :451-468) and the new cell indices.
 template <typename V>
-__global__ void move3(const __grid_constant__ Grid3 g, const __grid_constant__ BubbleParams bp, Bub3 b, const V vx,
-                      const V vy, const V vz, Scalars3* s) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= b.n) return;
+__device__ __forceinline__ void move3_one(const Grid3& g, const BubbleParams& bp, Bub3& b, const V& vx, const V& vy,
+                                          const V& vz, Scalars3* s, int n, int* s_box) {
   b.R_pn[n] = b.R_p[n];
   b.R_nn[n] = b.R_n[n];
   b.d1_R_n[n] = b.d1_R_p[n];
@@ -491,15 +516,37 @@ __global__ void move3(const __grid_constant__ Grid3 g, const __grid_constant__ B
   b.y[n] = y + uy * g.dt;
   b.z[n] = z + uz * g.dt;
   index3(g, b, n);
-  const int bin = bin3_of(f, b.ibnx[n], b.ibny[n], b.ibnz[n]);
-  if (bin != b.bin[n]) atomicOr(&s->moved, 1);
-  b.bin[n] = bin;
-  atomicMin(&s->box[0], b.ibnx[n]);
-  atomicMin(&s->box[1], b.ibny[n]);
-  atomicMin(&s->box[2], b.ibnz[n]);
-  atomicMax(&s->box[3], b.ibnx[n]);
-  atomicMax(&s->box[4], b.ibny[n]);
-  atomicMax(&s->box[5], b.ibnz[n]);
+  const int ix = b.ibnx[n], iy = b.ibny[n], iz = b.ibnz[n];
+  const int bin = bin3_of(f, ix, iy, iz);
+  if (bin != b.bin[n]) {
+    atomicOr(&s->moved, 1);
+    b.bin[n] = bin;
+  }
+  // The bubbles' box: over the warp, then the block, then one atomic each per block
+  // (six per bubble on the same words took most of the launch: 2 M bubbles 477 us).
+  const unsigned m = __activemask();
+  const int r[6] = {__reduce_min_sync(m, ix), __reduce_min_sync(m, iy), __reduce_min_sync(m, iz),
+                    __reduce_max_sync(m, ix), __reduce_max_sync(m, iy), __reduce_max_sync(m, iz)};
+  if ((threadIdx.x & 31) == __ffs(m) - 1) {
+    for (int q = 0; q < 3; q++) {
+      atomicMin(&s_box[q], r[q]);
+      atomicMax(&s_box[q + 3], r[q + 3]);
+    }
+  }
+}
+template <typename V>
+__global__ void __launch_bounds__(256) move3(const __grid_constant__ Grid3 g, const __grid_constant__ BubbleParams bp,
+                                             Bub3 b, const V vx, const V vy, const V vz, Scalars3* s) {
+  __shared__ int s_box[6];
+  if (threadIdx.x < 6) s_box[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
+  __syncthreads();
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < b.n) move3_one(g, bp, b, vx, vy, vz, s, n, s_box);
+  __syncthreads();
+  if (threadIdx.x < 3)
+    atomicMin(&s->box[threadIdx.x], s_box[threadIdx.x]);
+  else if (threadIdx.x < 6)
+    atomicMax(&s->box[threadIdx.x], s_box[threadIdx.x]);
 }
 
 // Counting sort of bubbles by bin (ascending bubble index within a bin).
@@ -626,6 +673,11 @@ __device__ __forceinline__ void contrib3(const Grid3& g, const BubbleParams& bp,
 }
 
 constexpr int kRpThreads3 = 128;
+// Resident blocks per SM the register budget is set for, as the 2-D radius kernel's.
+template <typename P>
+constexpr int radius3_min_blocks() {
+  return sizeof(typename P::T) == sizeof(double) ? 7 : 5;
+}
 
 // The radius solves: the reference scheme's sub-steps (rp_substep_full) or
 // the rk45 scheme (rk_attempt), from the state stored at the step's start,
@@ -634,7 +686,7 @@ constexpr int kRpThreads3 = 128;
 // pattern of the last solve's keeps that solve's results: every input of its
 // solve is unchanged.
 template <typename P, bool RK>
-__global__ void __launch_bounds__(kRpThreads3) radius3(const __grid_constant__ Grid3 g,
+__global__ void __launch_bounds__(kRpThreads3, RK ? 1 : radius3_min_blocks<P>()) radius3(const __grid_constant__ Grid3 g,
                                                        const __grid_constant__ BubbleParams bp, Bub3 b,
                                                        const typename P::S px, const typename P::S py,
                                                        const typename P::S pz, Scalars3* sc, int reuse,
@@ -754,52 +806,107 @@ struct Couple3Args {
   typename P::G fg, fgn;
   const int* start;
   const double* contrib;
-  int box[6];  // cells [box0, box3] x [box1, box4] x [box2, box5]
-  int gather;  // 1: void fraction from the bins; 0: keep fg
+  Tiles3 tiles;
+  const int* n_tiles;
   int pressure;
   const double* elem_p;
   unsigned long long* residual;
 };
 
-// Per cell of the box: the void fraction from the eight bins whose bubbles
+// One warp per tile: whether a bin that touches its cells holds bubbles (the bins
+// of a row of cells are contiguous runs of the bin starts), and the list of the tiles
+// that may hold void fraction.  Only the tiles [lo, lo + n) that the bubbles' and the
+// supports' boxes meet.
+struct TileRange {
+  int lo[3], n[3];
+};
+__global__ void __launch_bounds__(256) mark_tiles(const Frame3 f, const int* __restrict__ start, Tiles3 t,
+                                                  TileRange r, int coupling, int* __restrict__ n_tiles) {
+  const int q = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (q >= r.n[0] * r.n[1] * r.n[2]) return;
+  const int tile = t.at(r.lo[0] + q % r.n[0], r.lo[1] + q / r.n[0] % r.n[1], r.lo[2] + q / (r.n[0] * r.n[1]));
+  const int i0 = tile % t.nx * kTile3X, j0 = tile / t.nx % t.ny * kTile3Y, k0 = tile / (t.nx * t.ny) * kTile3Z;
+  const int bx0 = i0 - 1, bx1 = min(i0 + kTile3X - 1, f.X + 1);
+  bool some = false;
+  for (int c = lane; c < (kTile3Y + 1) * (kTile3Z + 1); c += 32) {
+    const int by = j0 - 1 + c % (kTile3Y + 1), bz = k0 - 1 + c / (kTile3Y + 1);
+    if (by > f.Y + 1 || bz > f.Z + 1) continue;
+    const int row = ((bz + 1) * (f.Y + 3) + (by + 1)) * (f.X + 3);
+    some = some || start[row + bx0 + 1] != start[row + bx1 + 2];
+  }
+  some = __any_sync(0xffffffffu, some);
+  if (lane != 0) return;
+  int last = t.last[tile];
+  if (some) t.last[tile] = last = coupling;
+  if (coupling - last <= kTileLife) t.list[atomicAdd(n_tiles, 1)] = tile;
+}
+
+// Per cell of the active tiles: the void fraction from the eight bins whose bubbles
 // touch it (their runs in order, bins in a fixed order), then the pressure
 // re-evaluation with it, the source forcing and the residual.
+//
+// A block takes a plane of a tile, a warp 32 cells of a row.  The bins that touch them are four
+// contiguous runs of the bin starts, so two starts per run tell the warp which of the
+// runs hold bubbles at all.  (One thread per cell of the supports' box, each with its
+// 16 bin starts, took 868 us on 384^3 with a Gaussian cloud, most of it in cells without
+// void fraction.)
 template <typename P>
-__global__ void __launch_bounds__(256) couple3(const __grid_constant__ Grid3 g, const Couple3Args<P> a) {
+__global__ void __launch_bounds__(256, 4) couple3(const __grid_constant__ Grid3 g, const Couple3Args<P> a) {
   using G = typename P::G;
   const Frame3& f = g.f;
-  const int i = a.box[0] + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = a.box[1] + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = a.box[2] + blockIdx.z;
   unsigned long long res = 0ull;
-  if (i <= a.box[3] && j <= a.box[4] && k <= a.box[5]) {
-    const long o = f.idx(i, j, k);
-    double fgv;
-    bool same = false;  // the FDTD pass's pressure is already this cell's final value
-    if (a.gather) {
-      fgv = 0.0;
-      for (int ci = 0; ci < 2; ci++)
-        for (int cj = 0; cj < 2; cj++)
-          for (int ck = 0; ck < 2; ck++) {
-            const int bx = i - ci, by = j - cj, bz = k - ck;
-            if (bx < -1 || by < -1 || bz < -1) continue;
-            const int c = ((bz + 1) * (f.Y + 3) + (by + 1)) * (f.X + 3) + (bx + 1);
-            const int slot = ci * 4 + cj * 2 + ck;
+  const int n = *a.n_tiles * kTile3Z;
+  for (int t = blockIdx.x; t < n; t += gridDim.x) {
+    const int tile = a.tiles.list[t / kTile3Z];
+    const int i0 = tile % a.tiles.nx * kTile3X, i = i0 + threadIdx.x;
+    const int j = tile / a.tiles.nx % a.tiles.ny * kTile3Y + threadIdx.y;
+    const int k = tile / (a.tiles.nx * a.tiles.ny) * kTile3Z + t % kTile3Z;
+    if (k <= f.Z + 1) {
+      bool some = false;
+      if (threadIdx.x < 4 && j <= f.Y + 1) {
+        const int by = j - (int)(threadIdx.x >> 1), bz = k - (int)(threadIdx.x & 1);
+        const int row = ((bz + 1) * (f.Y + 3) + (by + 1)) * (f.X + 3);
+        some = a.start[row + i0] != a.start[row + min(i0 + kTile3X - 1, f.X + 1) + 2];
+      }
+      // Bit cj * 2 + ck: the run of bins (.., j - cj, k - ck) holds bubbles.
+      const unsigned runs = __ballot_sync(0xffffffffu, some);
+      if (i > f.X + 1 || j > f.Y + 1) continue;
+      const long o = f.idx(i, j, k);
+      double fgv = 0.0;
+      if (runs) {
+        // The starts of bins i - 1, i, i + 1 of the four runs, all at once; then each
+        // bin's values four at a time, added in order (absent ones as zeros).
+        int st[4][3];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const int row = ((k - (r & 1) + 1) * (f.Y + 3) + (j - (r >> 1) + 1)) * (f.X + 3) + i;
+#pragma unroll
+          for (int c = 0; c < 3; c++) st[r][c] = runs >> r & 1u ? a.start[row + c] : 0;
+        }
+#pragma unroll
+        for (int ci = 0; ci < 2; ci++)
+#pragma unroll
+          for (int r = 0; r < 4; r++) {
+            const double* __restrict__ v = a.contrib + ci * 4 + r;
             double run = 0.0;
-            for (int q = a.start[c]; q < a.start[c + 1]; q++) run += a.contrib[8 * (long)q + slot];
+            for (int q = st[r][1 - ci]; q < st[r][2 - ci]; q += 4) {
+              double w[4];
+#pragma unroll
+              for (int d = 0; d < 4; d++) w[d] = q + d < st[r][2 - ci] ? v[8 * (long)(q + d)] : 0.0;
+#pragma unroll
+              for (int d = 0; d < 4; d++) run += w[d];
+            }
             fgv += run;
           }
+      }
       fgv = G::stored(fgv);
       // No bubble touches the cell and its void fraction was zero in the
       // prediction and the step before: the gathered value is the stored 0
       // and the pressure evaluation would repeat the FDTD pass's (no
       // void-fraction rate), so the cell is left as it is.
-      same = fgv == 0.0 && a.fg.get(o) == 0.0 && a.fgn.get(o) == 0.0;
-      if (!same) a.fg.put(o, fgv);
-    } else {
-      fgv = a.fg.get(o);
-    }
-    if (!same && a.pressure && i >= 1 && i <= f.X && j >= 1 && j <= f.Y && k >= 1 && k <= f.Z) {
+      if (fgv == 0.0 && a.fg.get(o) == 0.0 && a.fgn.get(o) == 0.0) continue;
+      a.fg.put(o, fgv);
+      if (!(a.pressure && i >= 1 && i <= f.X && j >= 1 && j <= f.Y && k >= 1 && k <= f.Z)) continue;
       const double h = void_half3(g, fgv, a.fgn.get(o));
       const long ox = o - 1, oy = o - f.pitch, oz = o - (long)(f.Y + 4) * f.pitch;
       const double s1x = (-a.vx.get(ox) + a.vx.get(o)) * g.rdx;
@@ -821,12 +928,11 @@ __global__ void __launch_bounds__(256) couple3(const __grid_constant__ Grid3 g, 
         a.py.put(o, qy);
         a.pz.put(o, qz);
       }
-      res = (unsigned long long)__double_as_longlong(fabs(old - p0new));
+      res = max(res, (unsigned long long)__double_as_longlong(fabs(old - p0new)));
     }
   }
-  const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
   for (int off = 16; off > 0; off >>= 1) res = max(res, __shfl_xor_sync(0xffffffffu, res, off));
-  if (lane == 0 && res) atomicMax(a.residual, res);
+  if (threadIdx.x == 0 && res) atomicMax(a.residual, res);
 }
 
 // Contributions of every bubble at its current radius (set-up).
@@ -1071,7 +1177,7 @@ struct Sim3Impl {
   int* lpt_order = nullptr;
   bool use_order = false;     // the order was built for this step's radius solves
   int rp_grid = 1;
-  int rp_grid_full = 1;  // one lane per bubble, up to 4 blocks per SM
+  int rp_grid_full = 1;  // one lane per bubble, up to the occupancy limit
   int rp_blocks_req = 0;  // crp_set_tuning (0: rp_grid_full)
   int supp[3][6];
   crp_stats stats{};
@@ -1139,6 +1245,11 @@ struct Sim3Impl {
       bin_start = carve<int>(nbins + 1, off, dry);
       bin_idx = carve<int>(std::max(n, 1), off, dry);
       bin_partial = carve<int>((nbins + d3::kScan - 1) / d3::kScan + 1, off, dry);
+      tiles.nx = (FX + 2 + d3::kTile3X - 1) / d3::kTile3X;
+      tiles.ny = (FY + 2 + d3::kTile3Y - 1) / d3::kTile3Y;
+      tiles.nz = (FZ + 2 + d3::kTile3Z - 1) / d3::kTile3Z;
+      tiles.last = carve<int>((size_t)tiles.nx * tiles.ny * tiles.nz, off, dry);
+      tiles.list = carve<int>((size_t)tiles.nx * tiles.ny * tiles.nz, off, dry);
       lpt_hist = carve<int>(kLptBuckets, off, dry);
       lpt_cursor = carve<int>(kLptBuckets, off, dry);
       lpt_order = carve<int>(n, off, dry);
@@ -1175,7 +1286,12 @@ struct Sim3Impl {
   template <typename P>
   crp_status launch_radius(int done);
   template <typename P>
-  crp_status launch_couple(bool gather, bool pressure, const int box[6]);
+  crp_status launch_couple(bool pressure);
+  d3::Tiles3 tiles{};
+  int64_t coupling = 0;  // couplings so far: steps whose Picard loop ran
+  // The active tiles of the next couplings of this step, from the current bins;
+  // now: the bubbles' box.
+  crp_status mark_tiles(const int now[6]);
   crp_status build_bins();
   crp_status build_order();
   cudaError_t begin_step(double t0, double t1) {
@@ -1463,11 +1579,16 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
     // buffers start equal to it.
     d3::contrib_init3<<<(nb + 255) / 256, 256, 0, stream>>>(g, bp, bub);
     C3(cudaGetLastError());
+    C3(cudaMemsetAsync(tiles.last, 0xc0, sizeof(int) * tiles.nx * tiles.ny * tiles.nz, stream));  // never touched
     C3(cudaMemcpyAsync(h_sc, d_sc, sizeof(d3::Scalars3), cudaMemcpyDeviceToHost, stream));
     C3(cudaStreamSynchronize(stream));
     int box[6];
     bubble_box(box);
-    const crp_status st = mixed ? launch_couple<d3::PMix>(true, false, box) : launch_couple<d3::P64>(true, false, box);
+    {
+      const crp_status ts = mark_tiles(box);
+      if (ts != CRP_OK) return ts;
+    }
+    const crp_status st = mixed ? launch_couple<d3::PMix>(false) : launch_couple<d3::P64>(false);
     if (st != CRP_OK) return st;
     const size_t bytes = sizeof(double) * cells;
     C3(cudaMemcpyAsync(fg[fg_b], fg[fg_a], bytes, cudaMemcpyDeviceToDevice, stream));
@@ -1476,7 +1597,15 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
   }
   int sms = 0;
   C3(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  rp_grid_full = std::max(1, std::min(sms * 4, (nb + d3::kRpThreads3 - 1) / d3::kRpThreads3));
+  int per_sm = 0;
+  const bool rk = c.ext_rp_scheme == CRP_RP_RK45;
+  if (mixed)
+    C3(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, rk ? d3::radius3<d3::PMix, true> : d3::radius3<d3::PMix, false>, d3::kRpThreads3, 0));
+  else
+    C3(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, rk ? d3::radius3<d3::P64, true> : d3::radius3<d3::P64, false>, d3::kRpThreads3, 0));
+  rp_grid_full = std::max(1, std::min(sms * std::max(per_sm, 1), (nb + d3::kRpThreads3 - 1) / d3::kRpThreads3));
   rp_grid = rp_grid_full;
   C3(cudaStreamSynchronize(stream));
   return CRP_OK;
@@ -1560,6 +1689,8 @@ crp_status Sim3Impl::launch_fdtd(const double* elem) {
   a.residual = &d_sc->residual;
   a.bubbles = bub.n > 0 ? 1 : 0;
   std::memcpy(a.supp, supp, sizeof(a.supp));
+  a.tiles = tiles;
+  a.coupling = (int)coupling + 1;
   a.elem_p = elem;
   const int sx = (g.f.X + d3::kCols3 - 1) / d3::kCols3, sy = (g.f.Y + d3::kRows3 - 1) / d3::kRows3;
   // Planes per chunk: up to 16 (256^3: 398 us, 425 with 32, 402 with 8), fewer where that
@@ -1626,12 +1757,31 @@ crp_status Sim3Impl::launch_radius(int done) {
   return CRP_OK;
 }
 
+crp_status Sim3Impl::mark_tiles(const int now[6]) {
+  int u[6], w[6], box[6];
+  box_union(u, now, supp[0]);
+  box_union(w, supp[1], supp[2]);
+  box_union(box, u, w);
+  C3(cudaMemsetAsync(&d_sc->tiles, 0, sizeof(int), stream));
+  if (box[0] > box[3] || box[1] > box[4] || box[2] > box[5]) return CRP_OK;
+  const int size[3] = {d3::kTile3X, d3::kTile3Y, d3::kTile3Z};
+  d3::TileRange r;
+  for (int q = 0; q < 3; q++) {
+    r.lo[q] = box[q] / size[q];
+    r.n[q] = box[q + 3] / size[q] - r.lo[q] + 1;
+  }
+  d3::mark_tiles<<<(r.n[0] * r.n[1] * r.n[2] + 7) / 8, 256, 0, stream>>>(g.f, bin_start, tiles, r, (int)coupling,
+                                                                          &d_sc->tiles);
+  C3(cudaGetLastError());
+  launches++;
+  return CRP_OK;
+}
+
 template <typename P>
-crp_status Sim3Impl::launch_couple(bool gather, bool pressure, const int box[6]) {
+crp_status Sim3Impl::launch_couple(bool pressure) {
   using V = typename P::V;
   using S = typename P::S;
   using G = typename P::G;
-  if (box[0] > box[3] || box[1] > box[4] || box[2] > box[5]) return CRP_OK;
   d3::Couple3Args<P> a;
   a.vx = view<V>(vx[cur_v]);
   a.vy = view<V>(vy[cur_v]);
@@ -1646,14 +1796,14 @@ crp_status Sim3Impl::launch_couple(bool gather, bool pressure, const int box[6])
   a.fgn = view<G>(fg[fg_b]);
   a.start = bin_start;
   a.contrib = bub.contrib;
-  for (int q = 0; q < 6; q++) a.box[q] = box[q];
-  a.gather = gather ? 1 : 0;
+  a.tiles = tiles;
+  a.n_tiles = &d_sc->tiles;
   a.pressure = pressure ? 1 : 0;
   a.elem_p = elem_p;
   a.residual = &d_sc->residual;
-  const dim3 block(32, 8);
-  const dim3 grid((box[3] - box[0] + 32) / 32, (box[4] - box[1] + 8) / 8, box[5] - box[2] + 1);
-  d3::couple3<P><<<grid, block, 0, stream>>>(g, a);
+  // The list's length is on the device: the blocks that the GPU holds stride over it.
+  const int grid = std::min(tiles.nx * tiles.ny * tiles.nz, 148 * 4);
+  d3::couple3<P><<<grid, dim3(32, 8), 0, stream>>>(g, a);
   C3(cudaGetLastError());
   launches++;
   return CRP_OK;
@@ -1737,12 +1887,13 @@ crp_status Sim3Impl::step_once() {
     bubble_box(bnow);
     if (h_sc->moved) bins_stale = true;
   }
-  int box[6], u1[6], u2[6];
-  box_union(u1, bnow, supp[0]);
-  box_union(u2, supp[1], supp[2]);
-  box_union(box, u1, u2);
-  if (bub.n > 0 && res > picard_tol && bins_stale) {
-    st = build_bins();
+  if (bub.n > 0 && res > picard_tol) {
+    if (bins_stale) {
+      st = build_bins();
+      if (st != CRP_OK) return st;
+    }
+    coupling++;
+    st = mark_tiles(bnow);
     if (st != CRP_OK) return st;
   }
   // Heaviest-first solve order from the last solves' sub-step counts, once
@@ -1759,7 +1910,7 @@ crp_status Sim3Impl::step_once() {
       C3(cudaMemsetAsync(&d_sc->residual, 0, sizeof(unsigned long long), stream));
       st = mixed ? launch_radius<d3::PMix>(loop - 1) : launch_radius<d3::P64>(loop - 1);
       if (st != CRP_OK) return st;
-      st = mixed ? launch_couple<d3::PMix>(true, true, box) : launch_couple<d3::P64>(true, true, box);
+      st = mixed ? launch_couple<d3::PMix>(true) : launch_couple<d3::P64>(true);
       if (st != CRP_OK) return st;
       C3(cudaMemcpyAsync(h_sc, d_sc, sizeof(d3::Scalars3), cudaMemcpyDeviceToHost, stream));
       C3(cudaStreamSynchronize(stream));
@@ -2088,6 +2239,7 @@ struct HostState3 {
   int cur_v, cur_p, fg_a, fg_b, fg_c, bins_stale;
   double tstep, tstepx, t_prev;
   int supp[3][6];
+  int64_t coupling;
   crp_stats stats;
   d3::Scalars3 hsc;
 };
@@ -2103,6 +2255,7 @@ crp_status sim3_save_state(Sim3Impl* s, void* blob, std::vector<unsigned char>& 
   std::memcpy(h.supp, s->supp, sizeof(h.supp));
   h.stats = s->stats;
   h.hsc = *s->h_sc;
+  h.coupling = s->coupling;
   host.resize(sizeof(HostState3));
   std::memcpy(host.data(), &h, sizeof(HostState3));
   return CRP_OK;
@@ -2118,6 +2271,7 @@ crp_status sim3_load_state(Sim3Impl* s, const void* blob, const std::vector<unsi
   s->bins_stale = h.bins_stale != 0;
   s->tstep = h.tstep, s->tstepx = h.tstepx, s->t_prev = h.t_prev;
   std::memcpy(s->supp, h.supp, sizeof(h.supp));
+  s->coupling = h.coupling;
   const crp_stats keep = s->stats;
   s->stats = h.stats;
   s->stats.kernel_launches = keep.kernel_launches;

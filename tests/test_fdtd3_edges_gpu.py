@@ -56,3 +56,19 @@ def test_with_a_cloud(shape, cloud, shape_kind):
         assert np.array_equal(gpu.bubbles("ibn_x"), cpu.bubbles("ibn_x"))
         r = cpu.bubbles("R_t")
         assert np.abs(gpu.bubbles("R_t") - r).max() <= TOL * r.max()
+
+
+def test_steps_without_coupling():
+    """A Picard tolerance so loose that the loop runs on some steps only: the void
+    fraction is extrapolated over gaps of up to 20 steps in between."""
+    cfg = grid(40, 22, 26, bubbles=200, ext_cloud_r=6e-4, ext_cloud_shape=1, tr_amp=0.02e6 / (998 * 1482),
+               ext_picard_tol=0.2, tr_on_wave=1, ext_ramp_cycles=0)
+    bub = crp.seed_bubbles3(cfg)
+    cpu = B.OracleSim3(cfg, bub)
+    with crp.Sim(cfg, bub) as gpu:
+        for n in (20, 30, 15, 35):
+            gpu.step(n)
+            cpu.step(n)
+            same(gpu, cpu, ("p0", "vx", "f_g", "f_gn", "f_gm"))
+            assert gpu.stats().picard_total == cpu.stats().picard_total
+        assert 20 < cpu.stats().picard_total < 130
