@@ -676,19 +676,22 @@ static __constant__ double kThermalB36[19] = {
 struct ThermalRatio {
   double Ar, Aj, Br, Bj;  // T = (Ar + i w Aj) / (Br + i w Bj)
 };
-// c[first] + c[first + 2] x + c[first + 4] x^2 + ... over the n coefficients of c.
+// c[first] + c[first + 2] x + c[first + 4] x^2 + ... over the N coefficients of c:
+// the even and the odd powers of x in two chains (x2 = x^2), half the latency of one.
 template <int N>
-__device__ __forceinline__ double every_other(const double (&c)[N], int first, double x) {
-  int k = N - 1 - ((N - 1 - first) & 1);
-  double v = c[k];
+__device__ __forceinline__ double every_other(const double (&c)[N], int first, double x, double x2) {
+  const int m = (N - 1 - first) / 2;  // highest power
+  double e = c[first + 2 * (m & ~1)], o = c[first + 2 * ((m - 1) | 1)];
 #pragma unroll
-  for (k -= 2; k >= first; k -= 2) v = fma(v, x, c[k]);
-  return v;
+  for (int k = (m & ~1) - 2; k >= 0; k -= 2) e = fma(e, x2, c[first + 2 * k]);
+#pragma unroll
+  for (int k = ((m - 1) | 1) - 2; k >= 1; k -= 2) o = fma(o, x2, c[first + 2 * k]);
+  return fma(o, x, e);
 }
 template <int N, int M>
 __device__ __forceinline__ ThermalRatio thermal_convergent(const double (&a)[N], const double (&b)[M], double w2) {
-  const double x = -w2;
-  return {every_other(a, 0, x), every_other(a, 1, x), every_other(b, 0, x), every_other(b, 1, x)};
+  const double x = -w2, x2 = w2 * w2;
+  return {every_other(a, 0, x, x2), every_other(a, 1, x, x2), every_other(b, 0, x, x2), every_other(b, 1, x, x2)};
 }
 __device__ __forceinline__ ThermalRatio thermal_ratio16(double w2) {
   return thermal_convergent(kThermalA16, kThermalB16, w2);
@@ -714,6 +717,7 @@ struct Thermal {
 // eta = (omega rho Rb)^2: w^2 = (2 coeff_alpha omega / Rb)^2 is proportional to it, T
 // depends on w^2, and Im(Upsilon) / (4 omega) on Im(Upsilon) / w, so each of the
 // three rounds takes one reciprocal and no square root.
+constexpr double kEtaFloor = 1.0e-6 * 2.22044604925031308e-016;
 struct ThermalPre {
   double base, c3, gq, ws2, caQ;
 };
@@ -723,17 +727,17 @@ __device__ __forceinline__ ThermalPre thermal_pre(const BubbleParams& b, double 
   const double caR = b.th_ca * pgr * inv_Rb;
   const double ws = 2.0 * caR * (b.inv_rho * inv_Rb);
   ThermalPre t;
-  t.base = b.th_base * inv_Rb;  // -2 sigma rho / Rb
+  t.base = __dmul_rn(b.th_base, inv_Rb);  // -2 sigma rho / Rb
   t.c3 = 4.0 * iR2;
-  t.gq = b.th_g3rho * Q;
+  t.gq = __dmul_rn(b.th_g3rho, Q);
   t.ws2 = ws * ws;
   t.caQ = caR * Q;
-  eta = larger(t.gq + t.base - b.mu * b.mu * t.c3, 1.0e-6 * 2.22044604925031308e-016);
+  eta = larger(fma(-(b.mu * b.mu), t.c3, t.gq + t.base), kEtaFloor);
   return t;
 }
 // eta from Re(Upsilon) / (3 gam) and the effective viscosity.
 __device__ __forceinline__ double thermal_eta(const ThermalPre& t, double ur, double mu_eff) {
-  return larger(fma(t.gq, ur, fma(-(mu_eff * t.c3), mu_eff, t.base)), 1.0e-6 * 2.22044604925031308e-016);
+  return larger(fma(t.gq, ur, fma(-(mu_eff * t.c3), mu_eff, t.base)), kEtaFloor);
 }
 __device__ __forceinline__ double thermal_round(const BubbleParams& b, const ThermalPre& t, const ThermalRatio& r,
                                                 double w2) {
@@ -776,42 +780,45 @@ static __device__ __noinline__ void thermal_any(const BubbleParams& b, double pg
 // about 20 um at rest), a compressed one, and a collapsed one (w >= 760), each valid
 // while all of its evaluations stay inside.  With coth(a) = 1 and d = 1 / s:
 // c / a^2 = (d - i d (1 - d)) / 2, and Lp's parts are polynomials in d.
-__device__ __forceinline__ Thermal thermal64(const BubbleParams& b, double pgr, double Rb, double inv_Rb) {
+// `beside` is called once in whichever range runs: work that does not depend on the
+// model, for a caller whose latency counts (its instructions are scheduled between
+// the rounds').  WIDE: all rounds unrolled.
+template <bool WIDE, typename F>
+__device__ __forceinline__ Thermal thermal64(const BubbleParams& b, double pgr, double Rb, double inv_Rb, F&& beside) {
   double eta;
   const ThermalPre t = thermal_pre(b, pgr, inv_Rb, eta);
   double w2 = t.ws2 * eta;
   Thermal o;
+  bool in = true;
   if (w2 < kThermalCut2) {
-    bool in = true;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       eta = thermal_round(b, t, thermal_ratio16(w2), w2);
       w2 = t.ws2 * eta;
       in = in && w2 < kThermalCut2;
+      if (k == 0) beside();
     }
     o = thermal_result(b, t, thermal_ratio16(w2), eta, w2, Rb, inv_Rb);
-    if (in) return o;
   } else if (w2 < kThermalLarge2) {
-    bool in = true;
-#pragma unroll 1
+#pragma unroll(WIDE ? 3 : 1)
     for (int k = 0; k < 3; k++) {
       eta = thermal_round(b, t, thermal_ratio36(w2), w2);
       w2 = t.ws2 * eta;
       in = in && w2 < kThermalLarge2;
+      if (k == 0) beside();
     }
     o = thermal_result(b, t, thermal_ratio36(w2), eta, w2, Rb, inv_Rb);
-    if (in) return o;
   } else {
-    bool in = true;
     double d = rroot4_pos(0.25 * w2);
-#pragma unroll 1
+#pragma unroll(WIDE ? 3 : 1)
     for (int k = 0; k < 3; k++) {
-      const double h = b.th_h * d, dr = 1.0 + h, di = fma(-h, d, h);
+      const double h = __dmul_rn(b.th_h, d), dr = 1.0 + h, di = fma(-h, d, h);
       const double inv = recip(fma(di, di, dr * dr));
       const double mu_eff = fma(b.th_kl * t.caQ * (d * d) * di, inv, b.mu);
       eta = thermal_eta(t, dr * inv, mu_eff);
       w2 = t.ws2 * eta;
       in = in && w2 >= kThermalLarge2;
+      if (k == 0) beside();
       d = rroot4_pos(0.25 * w2);
     }
     o.omega = b.inv_rho * inv_Rb * sqrt_pos(eta);
@@ -819,8 +826,8 @@ __device__ __forceinline__ Thermal thermal64(const BubbleParams& b, double pgr, 
     o.lr = 4.0 * e;
     o.li = fma(fma(fma(6.0, d, -12.0), d, 12.0), d, -4.0);
     o.den = Rb * d * fma(9.0 * de, de, f * f);
-    if (in) return o;
   }
+  if (in) return o;
   Thermal u;
   thermal_any(b, pgr, Rb, inv_Rb, &u);
   return u;

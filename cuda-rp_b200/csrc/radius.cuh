@@ -117,6 +117,11 @@ __device__ __forceinline__ Thermal thermal32(const ThermalConst<float>& c, doubl
   return {(double)omega, lr, li, lr * lr + li * li};
 }
 
+// a x + b y with every operation rounded.
+__device__ __forceinline__ double weighted(double a, double x, double b, double y) {
+  return __dadd_rn(__dmul_rn(a, x), __dmul_rn(b, y));
+}
+
 // One pass of the sub-step loop of BubbleRadiusKernel (:506-539):
 // solveRayleighPlesset (:227-260), one variable sub-step of the three-level
 // scheme; the thermal model at the old radius; solvePG (:326-340), with c1, c2, c3
@@ -128,51 +133,71 @@ __device__ __forceinline__ Thermal thermal32(const ThermalConst<float>& c, doubl
 // bubbles of 10 sub-steps takes 77 us, 178 us with the coth form) and by the latency of
 // this chain once a few bubbles are stiff (one sub-step alone on an SM: 1,080
 // cycles for w < 32, 1,450 to 1,630 above; the coth form 4,130 above).
-template <typename T>
+//
+// TIGHT: for launches that end with the chains of a few stiff bubbles.  The radius
+// update runs inside the thermal model's rounds, without branches of its own, and the
+// rounds are unrolled; the results are the same to the bit (every multiply-add is
+// written out, so that both are rounded alike).
+template <bool TIGHT, typename T>
 __device__ __forceinline__ void rp_substep_lean(const BubbleParams& b, RpState<T, kLean>& s) {
   const double eps = 2.22044604925031308e-016;
   const double PGn = s.PGp;
-  const double PL = s.PC2 * s.time * s.time + s.PC1 * s.time + s.PC0;
+  const double PL = fma(s.PC2 * s.time, s.time, fma(s.PC1, s.time, s.PC0));
   const double Rm = s.Rn, Rn = s.Rp, d1n = s.d1Rp;
   const double inv_Rn = recip(Rn);
+  const double dtm = s.dtL;
+  double dtp, Rp, d1, last;
+  auto radius = [&]() {
+    // The velocity and acceleration limits, 0.01 Rn / |d1R| and 0.1 Rn / sqrt(|acc|)
+    // (:238-241): each quotient is formed only where it is the smaller step, decided
+    // on the products (the squares for the second), so a quiet sub-step divides by
+    // neither.
+    const double net = fma(-(4.0 * b.mu * inv_Rn), d1n, fma(-2.0 * b.sig, inv_Rn, PGn - PL));
+    const double acc = fma(net, b.inv_rho, -__dmul_rn(1.5 * d1n, d1n));
+    dtp = smaller(1.01 * dtm, b.dt0);
+    const double ad = fabs(d1n), aa = fabs(acc), lim = 0.1 * Rn;
+    if (TIGHT) {
+      const double tv = 0.01 * Rn * recip(ad), ta = lim * rsqrt_pos(aa);
+      dtp = ad > eps && 0.01 * Rn < dtp * ad ? smaller(tv, dtp) : dtp;
+      dtp = aa > eps && lim * lim < dtp * dtp * aa ? smaller(ta, dtp) : dtp;
+    } else {
+      if (ad > eps && 0.01 * Rn < dtp * ad) dtp = smaller(0.01 * Rn * recip(ad), dtp);
+      if (aa > eps && lim * lim < dtp * dtp * aa) dtp = smaller(lim * rsqrt_pos(aa), dtp);
+    }
+    // q and 1 + q round as the reference's do: the rounding of 1 + q is the same at
+    // every sub-step of a constant growth and acts on R as a small force, 1e-9 of a
+    // driven bubble's radius after 1000 mixture steps.  So do the products of the
+    // velocity's difference, in which the radii cancel.
+    const double sum = dtm + dtp;
+    const double q = quotient(dtp, dtm);
+    const double inv3 = recip(dtm * dtp * sum);
+    const double tm2 = __dmul_rn(dtm, dtm), tp2 = __dmul_rn(dtp, dtp);  // their difference 0 at equal steps
+    Rp = fma(dtp * inv_Rn, 0.5 * sum * acc, fma(1.0 + q, Rn, -__dmul_rn(q, Rm)));
+    d1 = fma(__dadd_rn(weighted(tm2, Rp, tp2 - tm2, Rn), -__dmul_rn(tp2, Rm)), inv3, __dmul_rn(dtp * inv_Rn, acc));
+    s.Rt = Rp;
+    last = dtp;
+    if (TIGHT) {
+      const double rem = s.remain, qr = quotient(rem, dtm);
+      const double Rl = fma(rem * inv_Rn, 0.5 * (dtm + rem) * acc, fma(1.0 + qr, Rn, -__dmul_rn(qr, Rm)));
+      if (dtp >= rem) last = rem, s.Rt = Rl;
+    } else if (dtp >= s.remain) {
+      last = s.remain;
+      const double qr = quotient(last, dtm);
+      s.Rt = fma(last * inv_Rn, 0.5 * (dtm + last) * acc, fma(1.0 + qr, Rn, -__dmul_rn(qr, Rm)));
+    }
+  };
   Thermal th;
   if constexpr (sizeof(T) == sizeof(float)) {
     if (fabs(Rn - s.r.R0) > kThermalFp64Excursion * s.r.R0)
-      th = thermal64(b, s.r.c.pgr, Rn, inv_Rn);
+      th = thermal64<false>(b, s.r.c.pgr, Rn, inv_Rn, [] {});
     else
       th = thermal32(s.r.f, PGn, Rn);
+    radius();
+  } else if constexpr (TIGHT) {
+    th = thermal64<true>(b, s.r.c.pgr, Rn, inv_Rn, radius);
   } else {
-    th = thermal64(b, s.r.c.pgr, Rn, inv_Rn);
-  }
-  // Radius update.  The velocity and acceleration limits, 0.01 Rn / |d1R| and
-  // 0.1 Rn / sqrt(|acc|) (:238-241): each quotient is formed only where it is the
-  // smaller step, decided on the products (the squares for the second), so a
-  // quiet sub-step divides by neither.
-  const double acc =
-      (PGn - PL - 2.0 * b.sig * inv_Rn - 4.0 * b.mu * inv_Rn * d1n) * b.inv_rho - 1.5 * d1n * d1n;
-  const double dtm = s.dtL;
-  double dtp = smaller(1.01 * dtm, b.dt0);
-  const double ad = fabs(d1n), aa = fabs(acc);
-  if (ad > eps && 0.01 * Rn < dtp * ad) dtp = smaller(0.01 * Rn * recip(ad), dtp);
-  if (aa > eps) {
-    const double lim = 0.1 * Rn;
-    if (lim * lim < dtp * dtp * aa) dtp = smaller(lim * rsqrt_pos(aa), dtp);
-  }
-  // q and the products below round as the reference's do: the rounding of 1 + q is
-  // the same at every sub-step of a constant growth and acts on R as a small
-  // force, 1e-9 of a driven bubble's radius after 1000 mixture steps.
-  const double sum = dtm + dtp;
-  const double q = quotient(dtp, dtm);
-  const double inv3 = recip(dtm * dtp * sum);
-  const double Rp = (1.0 + q) * Rn - q * Rm + (dtp * inv_Rn) * (0.5 * sum * acc);
-  const double d1 =
-      (dtm * dtm * Rp + (-dtm * dtm + dtp * dtp) * Rn - dtp * dtp * Rm) * inv3 + (dtp * inv_Rn) * acc;
-  s.Rt = Rp;
-  double last = dtp;
-  if (dtp >= s.remain) {
-    last = s.remain;
-    const double qr = quotient(last, dtm);
-    s.Rt = (1.0 + qr) * Rn - qr * Rm + (last * inv_Rn) * (0.5 * (dtm + last) * acc);
+    th = thermal64<false>(b, s.r.c.pgr, Rn, inv_Rn, [] {});
+    radius();
   }
   s.remain -= last;
   s.Rn = Rn;
@@ -187,26 +212,27 @@ __device__ __forceinline__ void rp_substep_lean(const BubbleParams& b, RpState<T
   const double Rp3 = Rp * Rp * Rp, Rn3 = Rn * Rn * Rn;
   const double wd = th.omega * th.den;
   const double wh = th.omega * dtp * th.lr;
-  const double g = 0.5 * b.th_g3 * (Rp - Rn);
+  const double gd = Rp - Rn, gc = 0.5 * b.th_g3;
   const double a3 = 0.5 * k0 * wh * R3;
   const double wn = k0 * th.li;
-  const double c1 = wd * (R + g) + a3 - wn * Rp3;
-  const double c2 = wd * (R - g) - a3 - wn * Rn3;
-  const double PG = (c2 * PGn + k0 * wh * s.r.c.pgr) * recip(c1);
+  const double c1 = fma(-wn, Rp3, fma(wd, fma(gc, gd, R), a3));
+  const double c2 = fma(-wn, Rn3, fma(wd, fma(-gc, gd, R), -a3));
+  const double PG = fma(c2, PGn, __dmul_rn(k0 * wh, s.r.c.pgr)) * recip(c1);
   s.PGp = PG;
   // Heat flux (off the chain to the next sub-step) and viscous work:
   // 4 pi Rp^2 (4 mu d1R / Rp) d1R dt, with Rp^2 / Rp cancelled.
-  const double hx = wh * (s.r.c.pgr - 0.5 * (PG + PGn) * R3) + th.li * (PG * Rp3 - PGn * Rn3);
-  s.heat -= 4.0 * b.pi * Rp * Rp * b.K0 * (s.r.c.tpgr * hx * recip(wd));
-  s.vis += 4.0 * b.pi * Rp * 4.0 * b.mu * d1 * d1 * dtp;
+  const double hx = fma(wh, fma(-0.5 * (PG + PGn), R3, s.r.c.pgr),
+                        __dmul_rn(th.li, fma(PG, Rp3, -__dmul_rn(PGn, Rn3))));
+  s.heat = fma(-(4.0 * b.pi * b.K0 * Rp * Rp), s.r.c.tpgr * hx * recip(wd), s.heat);
+  s.vis = fma(16.0 * b.pi * b.mu * Rp * d1, d1 * dtp, s.vis);
 }
 
-template <typename T, int FORM>
+template <bool TIGHT, typename T, int FORM>
 __device__ __forceinline__ void rp_substep_full(const BubbleParams& b, RpState<T, FORM>& s) {
   if constexpr (FORM == kHeat)
     rp_substep_heat<T>(b, s);
   else
-    rp_substep_lean<T>(b, s);
+    rp_substep_lean<TIGHT, T>(b, s);
 }
 
 }  // namespace crp

@@ -617,16 +617,20 @@ __device__ __forceinline__ void store_contrib(const GridParams& g, const BubbleP
 // while the queue has work.  Each bubble's arithmetic is the same as a
 // thread-per-bubble solve, so results do not depend on the schedule.
 constexpr int kRpThreads = 128;
-// Resident blocks per SM the register budget is set for: 7 for the FP64 path
-// (at most 73 registers a thread), 5 for the mixed path (102): more warps to
-// hide the FP64 latency chains of the sub-step, measured faster than fewer
-// warps with more registers despite the spilled values (FP64, 1024 x 2048
-// quiet phase, per 100 steps: radius solve 17.2 ms at 7 blocks, 17.9 at 6,
-// 17.5 at 5; the mixed path's FP32 thermal model gains nothing from a sixth).
-template <typename P>
+// Resident blocks per SM the register budget is set for.  Quiet launches (TIGHT
+// false): 7 for the FP64 path (at most 73 registers a thread), 5 for the mixed path
+// (102): more warps to hide the FP64 latency chains of the sub-step, measured faster
+// than fewer warps with more registers despite the spilled values (FP64, 1024 x 2048,
+// 50 quiet steps: 10.77 ms at 7 blocks, 10.86 at 5, 11.18 at 4).  Launches that wait
+// for the chains of a few stiff bubbles (TIGHT): 3, nothing spilled.
+template <typename P, bool TIGHT>
 constexpr int rp_min_blocks() {
-  return sizeof(typename P::T) == sizeof(double) ? 7 : 5;
+  return TIGHT ? 3 : sizeof(typename P::T) == sizeof(double) ? 7 : 5;
 }
+// A launch counts as waiting for its stiffest bubble once one has needed this many
+// sub-steps (the quiet phase takes 10; 262,144 bubbles of 10 sub-steps take as long as
+// one bubble of about 150).
+constexpr long long kTightSubsteps = 150;
 
 // Lanes whose claimed bubble kept its last solve (n == -2) are counted, one
 // atomic per warp, and return to claiming (n = -1).  Called by the whole warp.
@@ -638,8 +642,8 @@ __device__ __forceinline__ void count_kept(int& n, unsigned long long* reused) {
   }
 }
 
-template <typename P, int FORM>
-__global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P>()) bubble_rp(const __grid_constant__ GridParams g,
+template <typename P, int FORM, bool TIGHT>
+__global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P, TIGHT>()) bubble_rp(const __grid_constant__ GridParams g,
                                                         const __grid_constant__ BubbleParams bp, BubbleArrays b,
                                                         const typename P::S px, const typename P::S py,
                                                         const double* __restrict__ tdev,
@@ -677,7 +681,7 @@ __global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P>()) bubble_rp(cons
     if (!__any_sync(0xffffffffu, n >= 0 || !drained)) break;
     if (n >= 0) {
       if (s.remain > 0.0 && s.count < bp.step_cap) {
-        rp_substep_full(bp, s);
+        rp_substep_full<TIGHT>(bp, s);
       } else {
         if (s.remain > 0.0) atomicOr(err, 1);
         rp_end(g, bp, b, n, s);
@@ -1529,6 +1533,7 @@ struct Sim {
     int* order;   // n
   } lpt{};
   int rp_grid = 1;
+  int rp_grid_tight = 1;      // the same of the kernel for launches with stiff bubbles
   int rp_grid_full = 1;       // the radius kernel's grid at one lane per bubble, up to the occupancy limit
   int couple_graph_grid = 1;  // blocks of the graph steps' coupling launch (striding over the box's tiles)
   // Launch tuning (crp_set_tuning): rows per FDTD strip chunk and the radius
@@ -1685,7 +1690,9 @@ struct Sim {
       int dev = 0, sms = 0, per_sm = 0;
       CRP_CUDA(cudaGetDevice(&dev));
       CRP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      CRP_CUDA(mixed ? radius_occupancy<PrecMixed>(&per_sm) : radius_occupancy<PrecFP64>(&per_sm));
+      CRP_CUDA(mixed ? radius_occupancy<PrecMixed>(&per_sm, true) : radius_occupancy<PrecFP64>(&per_sm, true));
+      rp_grid_tight = std::max(1, std::min(sms * std::max(per_sm, 1), (hs.nb + kRpThreads - 1) / kRpThreads));
+      CRP_CUDA(mixed ? radius_occupancy<PrecMixed>(&per_sm, false) : radius_occupancy<PrecFP64>(&per_sm, false));
       rp_grid_full = std::max(1, std::min(sms * std::max(per_sm, 1), (hs.nb + kRpThreads - 1) / kRpThreads));
       rp_grid = rp_grid_full;
       couple_graph_grid = 4 * sms;
@@ -2729,21 +2736,27 @@ struct Sim {
 
   // The radius kernel of this simulation: rk45, or the reference scheme in the
   // form its temperature branch asks for (RadiusForm).
+  // A graph's launches cannot choose by the sub-steps so far; they take the quiet one.
   template <typename P>
-  auto radius_kernel() const {
-    return cfg.ext_rp_scheme == CRP_RP_RK45 ? bubble_rk45<P> : temperature_on ? bubble_rp<P, kHeat> : bubble_rp<P, kLean>;
+  auto radius_kernel(bool tight) const {
+    return cfg.ext_rp_scheme == CRP_RP_RK45 ? bubble_rk45<P>
+           : temperature_on                 ? bubble_rp<P, kHeat, false>
+           : tight                          ? bubble_rp<P, kLean, true>
+                                            : bubble_rp<P, kLean, false>;
   }
   template <typename P>
-  cudaError_t radius_occupancy(int* per_sm) const {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, radius_kernel<P>(), kRpThreads, 0);
+  cudaError_t radius_occupancy(int* per_sm, bool tight) const {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, radius_kernel<P>(tight), kRpThreads, 0);
   }
   template <typename P>
   cudaError_t launch_rp() {
     using S = typename P::S;
     const S pxc = view<S>(px[cur_p]), pyc = view<S>(py[cur_p]);
-    const auto kernel = radius_kernel<P>();
+    const bool tight = !capturing && h_scalars->substep_max >= kTightSubsteps;
+    const auto kernel = radius_kernel<P>(tight);
+    const int grid = tight ? std::min(rp_grid, rp_grid_tight) : rp_grid;
     return launch(kClassRp, [&] {
-      kernel<<<rp_grid, kRpThreads, 0, stream>>>(gp, bp, bub, pxc, pyc, d_scalars->t, lpt.order, d_next, d_substep_max,
+      kernel<<<grid, kRpThreads, 0, stream>>>(gp, bp, bub, pxc, pyc, d_scalars->t, lpt.order, d_next, d_substep_max,
                                                  d_err, &d_scalars->loop, &d_scalars->reused);
     });
   }

@@ -673,11 +673,13 @@ __device__ __forceinline__ void contrib3(const Grid3& g, const BubbleParams& bp,
 }
 
 constexpr int kRpThreads3 = 128;
-// Resident blocks per SM the register budget is set for, as the 2-D radius kernel's.
-template <typename P>
+// Resident blocks per SM the register budget is set for, and the sub-step count from
+// which a launch waits for its stiffest bubble (TIGHT): as the 2-D radius kernel's.
+template <typename P, bool TIGHT>
 constexpr int radius3_min_blocks() {
-  return sizeof(typename P::T) == sizeof(double) ? 7 : 5;
+  return TIGHT ? 3 : sizeof(typename P::T) == sizeof(double) ? 7 : 5;
 }
+constexpr long long kTightSubsteps3 = 150;
 
 // The radius solves: the reference scheme's sub-steps (rp_substep_full) or
 // the rk45 scheme (rk_attempt), from the state stored at the step's start,
@@ -685,8 +687,8 @@ constexpr int radius3_min_blocks() {
 // this step has completed), a bubble whose gathered pressure has the bit
 // pattern of the last solve's keeps that solve's results: every input of its
 // solve is unchanged.
-template <typename P, bool RK>
-__global__ void __launch_bounds__(kRpThreads3, RK ? 1 : radius3_min_blocks<P>()) radius3(const __grid_constant__ Grid3 g,
+template <typename P, bool RK, bool TIGHT>
+__global__ void __launch_bounds__(kRpThreads3, RK ? 1 : radius3_min_blocks<P, TIGHT>()) radius3(const __grid_constant__ Grid3 g,
                                                        const __grid_constant__ BubbleParams bp, Bub3 b,
                                                        const typename P::S px, const typename P::S py,
                                                        const typename P::S pz, Scalars3* sc, int reuse,
@@ -775,7 +777,7 @@ __global__ void __launch_bounds__(kRpThreads3, RK ? 1 : radius3_min_blocks<P>())
       worst = max(worst, r.count);
     } else {
       if (s.remain > 0.0 && s.count < bp.step_cap) {
-        rp_substep_full(bp, s);
+        rp_substep_full<TIGHT>(bp, s);
         continue;
       }
       if (s.remain > 0.0) atomicOr(&sc->err, 1);
@@ -1177,6 +1179,7 @@ struct Sim3Impl {
   int* lpt_order = nullptr;
   bool use_order = false;     // the order was built for this step's radius solves
   int rp_grid = 1;
+  int rp_grid_tight = 1;  // the same of the kernel for launches with stiff bubbles
   int rp_grid_full = 1;  // one lane per bubble, up to the occupancy limit
   int rp_blocks_req = 0;  // crp_set_tuning (0: rp_grid_full)
   int supp[3][6];
@@ -1283,6 +1286,12 @@ struct Sim3Impl {
   crp_status launch_fdtd(const double* elem);
   template <typename P>
   crp_status launch_move();
+  template <typename P>
+  auto radius_kernel(bool tight) const {
+    return cfg.ext_rp_scheme == CRP_RP_RK45 ? d3::radius3<P, true, false>
+           : tight                          ? d3::radius3<P, false, true>
+                                            : d3::radius3<P, false, false>;
+  }
   template <typename P>
   crp_status launch_radius(int done);
   template <typename P>
@@ -1597,15 +1606,15 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
   }
   int sms = 0;
   C3(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  int per_sm = 0;
-  const bool rk = c.ext_rp_scheme == CRP_RP_RK45;
-  if (mixed)
-    C3(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, rk ? d3::radius3<d3::PMix, true> : d3::radius3<d3::PMix, false>, d3::kRpThreads3, 0));
-  else
-    C3(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, rk ? d3::radius3<d3::P64, true> : d3::radius3<d3::P64, false>, d3::kRpThreads3, 0));
-  rp_grid_full = std::max(1, std::min(sms * std::max(per_sm, 1), (nb + d3::kRpThreads3 - 1) / d3::kRpThreads3));
+  for (int tight = 0; tight < 2; tight++) {
+    int per_sm = 0;
+    if (mixed)
+      C3(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, radius_kernel<d3::PMix>(tight), d3::kRpThreads3, 0));
+    else
+      C3(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, radius_kernel<d3::P64>(tight), d3::kRpThreads3, 0));
+    (tight ? rp_grid_tight : rp_grid_full) =
+        std::max(1, std::min(sms * std::max(per_sm, 1), (nb + d3::kRpThreads3 - 1) / d3::kRpThreads3));
+  }
   rp_grid = rp_grid_full;
   C3(cudaStreamSynchronize(stream));
   return CRP_OK;
@@ -1745,13 +1754,11 @@ crp_status Sim3Impl::launch_radius(int done) {
   const int reuse = bp.reuse && done > 0 ? 1 : 0;
   const int* order = use_order ? lpt_order : nullptr;
   C3(cudaMemsetAsync(&d_sc->next, 0, sizeof(int), stream));
-  if (cfg.ext_rp_scheme == CRP_RP_RK45)
-    d3::radius3<P, true><<<rp_grid, d3::kRpThreads3, 0, stream>>>(g, bp, bub, view<S>(px[cur_p]), view<S>(py[cur_p]),
-                                                                   view<S>(pz[cur_p]), d_sc, reuse, order);
-  else
-    d3::radius3<P, false><<<rp_grid, d3::kRpThreads3, 0, stream>>>(g, bp, bub, view<S>(px[cur_p]),
-                                                                    view<S>(py[cur_p]), view<S>(pz[cur_p]), d_sc, reuse,
-                                                                    order);
+  const bool tight = h_sc->substep_max >= d3::kTightSubsteps3;
+  const auto kernel = radius_kernel<P>(tight);
+  const int grid = tight && cfg.ext_rp_scheme != CRP_RP_RK45 ? std::min(rp_grid, rp_grid_tight) : rp_grid;
+  kernel<<<grid, d3::kRpThreads3, 0, stream>>>(g, bp, bub, view<S>(px[cur_p]), view<S>(py[cur_p]), view<S>(pz[cur_p]),
+                                               d_sc, reuse, order);
   C3(cudaGetLastError());
   launches++;
   return CRP_OK;

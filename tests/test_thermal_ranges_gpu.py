@@ -49,3 +49,23 @@ def test_thermal_range_matches_oracle(name, scheme):
     print(name, scheme, errs)
     assert np.max(np.abs(cpu.bubbles("R_t") / r0 - 1.0)) > 1e-7  # the burst has reached the bubbles
     assert max(errs.values()) < TOL, errs
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_stiff_launches_round_as_quiet_ones(precision):
+    """A cloud that starts to collapse (1,468 sub-steps): host-driven steps take the
+    radius kernel for stiff launches once a bubble has needed 150 sub-steps, graph
+    steps the quiet one throughout; bit for bit the same."""
+    out = []
+    for graphs in (0, 1):
+        cfg = B.small_config(tr_amp=0.2, dbg_T=0, ext_bubble_count=120, ext_bubble_seed=3, ext_r0_sigma_ln=0.3,
+                             ext_cloud_r=8e-4, ext_cloud_h=2e-3, ext_n_b=1.0, bub_R0=3e-6, ext_precision=precision,
+                             ext_graphs=graphs)
+        bub = crp.seed_bubbles(cfg)
+        with crp.Sim(cfg, bub) as gpu:
+            gpu.step(290)
+            gpu.step(25)
+            assert gpu.stats().rp_substeps_max > 1000
+            out.append([gpu.field(k) for k in ("p0", "vx", "f_g")] + [gpu.bubbles(k) for k in ("R_t", "PG_p", "Q_B")])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
