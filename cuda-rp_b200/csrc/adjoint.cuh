@@ -15,12 +15,19 @@
 // sum_n dt sum_focal w p0^2 adds 2 dt w p0^n to both component adjoints at
 // every step, from the focal pressures the forward recorded (adj_record).
 //
-// adj_step does all of one reverse step in one pass: each cell forms the Lt
-// of the four faces it reads (its east and north faces, and its west and south
-// faces, which its neighbours form too, by the same expression) from the
-// previous step's L and M, and writes the next step's L and M into the other
-// of two frame sets.  Per cell and step it reads 4 doubles (L_x, L_y, M_x, M_y;
-// the neighbours' values come through L1/L2) and writes 4: 64 bytes.
+// adj_march does all of one reverse step in one pass, organised as fdtd_march: a
+// warp covers 64 columns, two per lane, and marches up a few rows.  A lane forms the
+// Lt of the three x faces and the north faces of its columns from the previous step's
+// L and M (the faces shared with other lanes twice, by the same expression; the south
+// faces are the north faces of the row below) and writes the next step's L and M into
+// the other of two frame sets.  The column coefficients stay in registers over the
+// chunk's rows, and the source's derivatives come from a table (source_derivative_rows),
+// so the pass carries no transcendental code.  Per cell and step it reads 4 doubles
+// (L_x, L_y, M_x, M_y; the neighbours' values come through L1/L2) and writes 4: 64 bytes.
+// Bound by the latency of the loads at 16 warps per SM: 600 x 701 takes 11.6 us cold
+// (27 MB: 2.3 TB/s).  A call of 200 steps there takes 7.5 ms; 8.2 with one cell per
+// thread, each reading the coefficients of its row and column again and evaluating
+// the source's derivatives where the source row lies.
 #pragma once
 #include "crp_device.cuh"
 
@@ -59,36 +66,6 @@ __device__ __forceinline__ double adj_kx_west(const GridParams& g, int c) {
   return g.cyl ? g.xu[c] * g.rdx * g.rxp[c] : g.rdx;
 }
 
-// Transpose of the pressure update at one face: Lt = L + (d p' / d v')^T M.
-// x face i (0 <= i <= X) of row j (1 <= j <= Y): east face of cell i, west
-// face of cell i+1.
-__device__ __forceinline__ double adj_lxt(const GridParams& g, const AdjFrames& a, int i, int j) {
-  const Frame& f = g.f;
-  double v = a.LX[f.idx(i, j)];
-  if (i >= 1) v -= g.s3p * g.pbx[i] * adj_kx_east(g, i) * a.MX[f.idx(i, j)];
-  if (i + 1 <= f.X) v += g.s3p * g.pbx[i + 1] * adj_kx_west(g, i + 1) * a.MX[f.idx(i + 1, j)];
-  return v;
-}
-// y face j (0 <= j <= Y) of column i (1 <= i <= X): north face of row j,
-// south face of row j+1.
-__device__ __forceinline__ double adj_lyt(const GridParams& g, const AdjFrames& a, int i, int j) {
-  const Frame& f = g.f;
-  double v = a.LY[f.idx(i, j)];
-  if (j >= 1) v -= g.s3p * g.pby[j] * g.rdy * a.MY[f.idx(i, j)];
-  if (j + 1 <= f.Y) v += g.s3p * g.pby[j + 1] * g.rdy * a.MY[f.idx(i, j + 1)];
-  return v;
-}
-
-// Gradient share of one source value: L (its adjoint) times its derivatives.
-__device__ __forceinline__ void adj_source_grad(const GridParams& g, const AdjGrad& gr, int i, double ym,
-                                                double t_src, double L) {
-  if (g.elem_n == 0) return;  // no elements: J only
-  double dA, dP;
-  source_derivatives(g, ((double)i - 0.5) * g.dx, ym, t_src, dA, dP);
-  gr.gA[i] += L * dA;
-  gr.gP[i] += L * dP;
-}
-
 // Focal box: cells [bi0, bi0 + bw) x [bj0, bj0 + bh), weights w (0 outside
 // the focal disk and on the source row).
 struct FocalBox {
@@ -96,60 +73,158 @@ struct FocalBox {
   const double* w;
 };
 
+// Derivatives of the source's row (source_derivatives) at the times of up to
+// kDerivBatch reverse steps: rows of X + 2 values, d / d amplitude then d / d phase of
+// each step.
+constexpr int kDerivBatch = 32;
+struct DerivTimes {
+  double t[kDerivBatch];
+};
+__global__ void __launch_bounds__(64) source_derivative_rows(const __grid_constant__ GridParams g,
+                                                             const __grid_constant__ DerivTimes d, double* out) {
+  const int i = blockIdx.x * 64 + threadIdx.x, w = g.f.X + 2;
+  if (i < 1 || i > g.f.X) return;
+  double dA, dP;
+  source_derivatives(g, ((double)i - 0.5) * g.dx, ((double)g.source_row - 0.5) * g.dy, d.t[blockIdx.y], dA, dP);
+  out[(2 * (size_t)blockIdx.y) * w + i] = dA;
+  out[(2 * (size_t)blockIdx.y + 1) * w + i] = dP;
+}
+
+constexpr int kAdjWarps = 4;
+
 // One reverse step: the transposes of the pressure update, the velocity update
-// and p0, from `in` into `out`; t_src is the time of the source values that
-// step read.  p0 (the focal pressures of the step before, or null for the
-// first step) adds that step's objective term.  Threads over the cells
-// [1, X] x [1, Y]; the cells of column 1 and row 1 also write the x0 and y0
-// face adjoints.
-__global__ void adj_step(const __grid_constant__ GridParams g, const AdjFrames in, const AdjFrames out,
-                         const AdjGrad gr, double t_src, const FocalBox b, const double* __restrict__ p0) {
+// and p0, from `in` into `out`; dA, dP: the source derivatives of the values that the
+// step read (null without elements).  p0 (the focal pressures of the step before, or
+// null for the first step) adds that step's objective term.
+__global__ void __launch_bounds__(32 * kAdjWarps, 4) adj_march(const __grid_constant__ GridParams g, const AdjFrames in,
+                                                               const AdjFrames out, const AdjGrad gr,
+                                                               const double* __restrict__ dA,
+                                                               const double* __restrict__ dP, const FocalBox b,
+                                                               const double* __restrict__ p0, int rows, int strips) {
   const Frame& f = g.f;
   const int X = f.X, Y = f.Y;
-  const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-  if (i > X || j > Y) return;
-  const long k = f.idx(i, j);
-  const double xe = adj_lxt(g, in, i, j), xw = adj_lxt(g, in, i - 1, j);
-  const double yn = adj_lyt(g, in, i, j), ys = adj_lyt(g, in, i, j - 1);
-  // Adjoint of p0(i, j): the faces that read it.
-  double L0 = 0.0;
-  if (adj_xface_on(g, i)) L0 += adj_cx(g, i) * xe;
-  if (adj_xface_on(g, i - 1)) L0 -= adj_cx(g, i - 1) * xw;
-  if (adj_yface_on(g, j)) L0 += adj_cy(g, j) * yn;
-  if (adj_yface_on(g, j - 1)) L0 -= adj_cy(g, j - 1) * ys;
-  if (j == 1 && !g.pml_y0) {
-    // The y0 face also reads the ghost value p0(i, 0): the source on the ghost
-    // row (source_row 0), else the mirror of p0(i, 1).
-    const double m = adj_cy(g, 0) * ys;
-    if (g.source_row == 0)
-      adj_source_grad(g, gr, i, -0.5 * g.dy, t_src, m);
-    else
-      L0 += m;
+  const int i = 1 + (blockIdx.x % strips) * 64 + 2 * (threadIdx.x & 31);
+  const int j0 = 1 + ((blockIdx.x / strips) * kAdjWarps + (threadIdx.x >> 5)) * rows, j1 = min(Y, j0 + rows - 1);
+  if (i > X || j0 > Y) return;
+  const bool two = i + 1 <= X;
+  const unsigned pitch = (unsigned)f.pitch;
+  auto get2 = [](const double* p, unsigned k) { return *reinterpret_cast<const double2*>(p + k); };
+  // Column coefficients of the faces i - 1, i, i + 1: the pressure update's weights of
+  // the cells west (cw) and east (ce) of the face, d v' / d p0, and d v' / d v.
+  double cw[3], ce[3], cx[3], ax[3];
+  bool on[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const int q = min(i - 1 + c, X);
+    on[c] = adj_xface_on(g, q);
+    cw[c] = q >= 1 ? g.s3p * g.pbx[q] * adj_kx_east(g, q) : 0.0;
+    ce[c] = q + 1 <= X ? g.s3p * g.pbx[q + 1] * adj_kx_west(g, q + 1) : 0.0;
+    cx[c] = adj_cx(g, q);
+    ax[c] = adj_ax(g, q);
   }
-  double mx = in.MX[k], my = in.MY[k];
-  if (g.source_row > 0 && j == g.source_row) {
-    adj_source_grad(g, gr, i, ((double)g.source_row - 0.5) * g.dy, t_src, L0);
-  } else {
-    mx = g.pax[i] * mx + L0;
-    my = g.pay[j] * my + L0;
-  }
-  if (p0) {  // d J / d p0 of the step before: M += 2 dt w p0 on the focal box
-    const int bi = i - b.bi0, bj = j - b.bj0;
-    if (bi >= 0 && bi < b.bw && bj >= 0 && bj < b.bh) {
-      const int q = bj * b.bw + bi;
-      const double v = 2.0 * g.dt * b.w[q] * p0[q];
-      mx += v;
-      my += v;
+  const double pax[2] = {g.pax[i], g.pax[min(i + 1, X)]};
+  unsigned k = (unsigned)(j0 + 1) * pitch + (unsigned)(i + 1);
+  // Lt of the south faces (adj_lyt of row j0 - 1).
+  double ys[2];
+  double2 my = get2(in.MY, k);
+  {
+    const double2 l = get2(in.LY, k - pitch), m = get2(in.MY, k - pitch);
+    const double lv[2] = {l.x, l.y}, mb[2] = {m.x, m.y}, mc[2] = {my.x, my.y};
+    const double wb = j0 >= 2 ? g.s3p * g.pby[j0 - 1] * g.rdy : 0.0, wt = g.s3p * g.pby[j0] * g.rdy;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      ys[c] = lv[c];
+      if (j0 >= 2) ys[c] = fma(-wb, mb[c], ys[c]);
+      ys[c] = fma(wt, mc[c], ys[c]);
     }
   }
-  out.MX[k] = mx;
-  out.MY[k] = my;
-  // Face adjoints one step back (each cell takes its east and north faces; the
-  // first column and row also the x0 and y0 faces).
-  out.LX[k] = adj_xface_on(g, i) ? adj_ax(g, i) * xe : 0.0;
-  if (i == 1) out.LX[f.idx(0, j)] = adj_xface_on(g, 0) ? adj_ax(g, 0) * xw : 0.0;
-  out.LY[k] = adj_yface_on(g, j) ? adj_ay(g, j) * yn : 0.0;
-  if (j == 1) out.LY[f.idx(i, 0)] = adj_ay(g, 0) * ys;
+  for (int j = j0; j <= j1; j++, k += pitch) {
+    const double2 lx = get2(in.LX, k), ly = get2(in.LY, k), mx = get2(in.MX, k), mn = get2(in.MY, k + pitch);
+    const double lw = in.LX[k - 1], mw = in.MX[k - 1], me = in.MX[k + 2];
+    const double m4[4] = {mw, mx.x, mx.y, me}, l3[3] = {lw, lx.x, lx.y};
+    double xt[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double v = l3[c];
+      if (i - 1 + c >= 1) v = fma(-cw[c], m4[c], v);
+      if (i + c <= X) v = fma(ce[c], m4[c + 1], v);
+      xt[c] = v;
+    }
+    const double wb = g.s3p * g.pby[j] * g.rdy, wt = j + 1 <= Y ? g.s3p * g.pby[j + 1] * g.rdy : 0.0;
+    const double cyn = adj_cy(g, j), cys = adj_cy(g, j - 1), ayn = adj_ay(g, j), pay = g.pay[j];
+    const bool on_n = adj_yface_on(g, j), on_s = adj_yface_on(g, j - 1);
+    const double lyv[2] = {ly.x, ly.y}, myv[2] = {my.x, my.y}, mnv[2] = {mn.x, mn.y};
+    double yn[2], nmx[2], nmy[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      yn[c] = fma(-wb, myv[c], lyv[c]);
+      if (j + 1 <= Y) yn[c] = fma(wt, mnv[c], yn[c]);
+      // Adjoint of p0(i + c, j): the faces that read it.
+      double L0 = 0.0;
+      if (on[c + 1]) L0 = fma(cx[c + 1], xt[c + 1], L0);
+      if (on[c]) L0 = fma(-cx[c], xt[c], L0);
+      if (on_n) L0 = fma(cyn, yn[c], L0);
+      if (on_s) L0 = fma(-cys, ys[c], L0);
+      if (c == 1 && !two) break;
+      const int col = i + c;
+      if (j == 1 && !g.pml_y0) {
+        // The y0 face also reads the ghost value p0(i, 0): the source on the ghost
+        // row (source_row 0), else the mirror of p0(i, 1).
+        const double m = __dmul_rn(adj_cy(g, 0), ys[c]);
+        if (g.source_row == 0) {
+          if (dA) {
+            gr.gA[col] += m * dA[col];
+            gr.gP[col] += m * dP[col];
+          }
+        } else {
+          L0 += m;
+        }
+      }
+      double ux = m4[c + 1], uy = myv[c];
+      if (g.source_row > 0 && j == g.source_row) {
+        if (dA) {
+          gr.gA[col] += L0 * dA[col];
+          gr.gP[col] += L0 * dP[col];
+        }
+      } else {
+        ux = fma(pax[c], ux, L0);
+        uy = fma(pay, uy, L0);
+      }
+      if (p0) {  // d J / d p0 of the step before: M += 2 dt w p0 on the focal box
+        const int bi = col - b.bi0, bj = j - b.bj0;
+        if (bi >= 0 && bi < b.bw && bj >= 0 && bj < b.bh) {
+          const int q = bj * b.bw + bi;
+          const double v = __dmul_rn(2.0 * g.dt * b.w[q], p0[q]);
+          ux += v;
+          uy += v;
+        }
+      }
+      nmx[c] = ux;
+      nmy[c] = uy;
+    }
+    // Face adjoints one step back (each cell takes its east and north faces; the
+    // first column and row also the x0 and y0 faces).
+    const double fx[2] = {on[1] ? ax[1] * xt[1] : 0.0, on[2] ? ax[2] * xt[2] : 0.0};
+    const double fy[2] = {on_n ? ayn * yn[0] : 0.0, on_n ? ayn * yn[1] : 0.0};
+    auto put = [&](double* q, double v, double w) {
+      if (two)
+        *reinterpret_cast<double2*>(q + k) = make_double2(v, w);
+      else
+        q[k] = v;
+    };
+    put(out.MX, nmx[0], nmx[1]);
+    put(out.MY, nmy[0], nmy[1]);
+    put(out.LX, fx[0], fx[1]);
+    put(out.LY, fy[0], fy[1]);
+    if (i == 1) out.LX[k - 1] = on[0] ? ax[0] * xt[0] : 0.0;
+    if (j == 1) {
+      out.LY[k - pitch] = adj_ay(g, 0) * ys[0];
+      if (two) out.LY[k - pitch + 1] = adj_ay(g, 0) * ys[1];
+    }
+    ys[0] = yn[0];
+    ys[1] = yn[1];
+    my = mn;
+  }
 }
 
 // p0 of the focal box after a forward step (interior cells: px + py).
@@ -163,7 +238,7 @@ __global__ void adj_record(const __grid_constant__ GridParams g, const S px, con
 }
 
 // d J / d p0 of the last step: MX, MY += 2 dt w p0 (the earlier steps' terms
-// are added by adj_step).
+// are added by adj_march).
 __global__ void adj_force(const __grid_constant__ GridParams g, const AdjFrames a, const FocalBox b,
                           const double* __restrict__ p0) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;

@@ -3044,7 +3044,7 @@ cudaError_t Sim::launch_couple_t(bool pressure) {
 }
 
 // crp_adjoint: obj->steps forward steps recording the focal p0, the
-// objective, then the reverse sweep (adj_force for the last step, one adj_step
+// objective, then the reverse sweep (adj_force for the last step, one adj_march
 // per step, adjoint.cuh) and the per-element sums of the per-column gradients.
 crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, double* grad_phase) {
   if (!obj || obj->steps <= 0 || !(obj->focal_radius > 0.0))
@@ -3082,7 +3082,8 @@ crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, d
   const size_t hist_n = (size_t)N * cells_box;
   if (hist_n * sizeof(double) > ((size_t)32 << 30))
     return fail(CRP_ERR_TOO_LARGE, "adjoint: focal history above 32 GiB (steps x focal cells)");
-  const size_t n_doubles = 8 * cells + 2 * (size_t)(X + 2) + cells_box + hist_n + (size_t)N;
+  const size_t n_der = 2 * (size_t)kDerivBatch * (X + 2);
+  const size_t n_doubles = 8 * cells + 2 * (size_t)(X + 2) + cells_box + hist_n + (size_t)N + n_der;
   double* buf = nullptr;
   {
     const crp_status ws = adjoint_workspace(n_doubles * sizeof(double), reinterpret_cast<void**>(&buf));
@@ -3103,6 +3104,7 @@ crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, d
   double* d_w = gr.gP + (X + 2);
   double* hist = d_w + cells_box;
   double* d_Jn = hist + hist_n;
+  double* der = d_Jn + N;  // source derivatives of a batch of reverse steps
   CRP_CUDA(cudaMemsetAsync(buf, 0, n_doubles * sizeof(double), stream));
   CRP_CUDA(cudaMemcpyAsync(d_w, w.data(), sizeof(double) * cells_box, cudaMemcpyHostToDevice, stream));
   const FocalBox box{bi0, bj0, bw, bh, d_w};
@@ -3142,14 +3144,26 @@ crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, d
   for (int n = 0; n < N; n++) Jsum += Jn[n];
   if (J) *J = gp.dt * Jsum;
   // Reverse sweep: reverse step n reads frame set s and writes set s ^ 1.
-  const dim3 blk(32, 8), gcells((X + 31) / 32, (Y + 7) / 8);
+  const int strips = (X + 63) / 64, rows = march_rows(strips);
+  const int grid = strips * (((Y + rows - 1) / rows + kAdjWarps - 1) / kAdjWarps);
   CRP_CUDA(launch(kClassOther, [&] { adj_force<<<rb, 256, 0, stream>>>(gp, fr[0], box, hist + (size_t)(N - 1) * cells_box); }));
   int s = 0;
   for (int n = N; n >= 1; n--, s ^= 1) {
-    const double t_src = times[n - 1];
+    // The source values that step n read are those of the time before it.
+    const int q = (N - n) % kDerivBatch;
+    if (gp.elem_n > 0 && q == 0) {
+      DerivTimes dt{};
+      const int m = std::min(n, kDerivBatch);
+      for (int r = 0; r < m; r++) dt.t[r] = times[n - 1 - r];
+      const dim3 dg((X + 64) / 64, m);
+      CRP_CUDA(launch(kClassOther, [&] { source_derivative_rows<<<dg, 64, 0, stream>>>(gp, dt, der); }));
+    }
+    const double* dA = gp.elem_n > 0 ? der + 2 * (size_t)q * (X + 2) : nullptr;
+    const double* dP = gp.elem_n > 0 ? dA + (X + 2) : nullptr;
     const double* p0 = n >= 2 ? hist + (size_t)(n - 2) * cells_box : nullptr;
-    CRP_CUDA(launch(kClassOther,
-                    [&] { adj_step<<<gcells, blk, 0, stream>>>(gp, fr[s], fr[s ^ 1], gr, t_src, box, p0); }));
+    CRP_CUDA(launch(kClassOther, [&] {
+      adj_march<<<grid, 32 * kAdjWarps, 0, stream>>>(gp, fr[s], fr[s ^ 1], gr, dA, dP, box, p0, rows, strips);
+    }));
   }
   if (gp.elem_n > 0) {
     std::vector<double> gA(X + 2), gPh(X + 2);

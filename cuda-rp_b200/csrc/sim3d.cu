@@ -993,16 +993,15 @@ struct PMix {
 // with p0 = px + py + pz (0 in the ghost cells, which are never written).  The
 // reverse of one step, given the adjoint of the state after it:
 //   1. adj3_source: the source cells' share of the gradient, their adjoint zeroed;
-//   2. adj3_step, one pass from one set of adjoint frames into the other:
+//   2. adj3_march, one pass from one set of adjoint frames into the other:
 //      the face adjoints take the pressure update's transpose; the component
 //      adjoints become pa_c M_c plus the velocity update's transpose into p0
 //      (the same for all three components); the face adjoints are multiplied
 //      by va vb; and 2 dt w p0 of the step before is added for the focal cells
 //      (adj3_force adds the last step's before the sweep).
-// Each cell forms the transposed values of its six faces (its west, south and
-// bottom faces by the same expression as the neighbour that owns them), so a
-// step reads 6 doubles per cell (L and M; neighbours through L1/L2) and
-// writes 6: 96 bytes.
+// Each cell forms the transposed values of its faces (its west and south faces by the
+// same expression as the neighbour that owns them), so a step reads 6 doubles per
+// cell (L and M; neighbours through L1/L2) and writes 6: 96 bytes.
 struct Adj3 {
   double *LX, *LY, *LZ;  // adjoints of vx, vy, vz (frame layout)
   double *MX, *MY, *MZ;  // adjoints of px, py, pz
@@ -1050,12 +1049,36 @@ __global__ void adj3_force(const Frame3 f, const Adj3 a, const Box3 b, const dou
   a.MZ[q] += d;
 }
 
-// Source cell c (frame index cells[c], element elem[c]) at the step's time t:
-// d p'_x / d amp_e and d p'_x / d phase_e times the adjoint of p'_x, summed
+// The source's factors at the times of up to kElemBatch reverse steps: whether the
+// burst is on, the envelope, every element's sine and cosine.
+struct SourceFactors {
+  double* env;  // [step][on, envelope]
+  double* sn;   // [step][element]
+  double* cs;
+};
+__global__ void __launch_bounds__(kBeginThreads3) adj3_factors(const __grid_constant__ Grid3 g,
+                                                               const __grid_constant__ ElemTimes s, int elems,
+                                                               const SourceFactors o) {
+  const int e = blockIdx.x * kBeginThreads3 + threadIdx.x;
+  const double t = s.t[blockIdx.y], tau = fmod(t, g.period);
+  if (e == 0) {
+    const bool on = t > 0.0 && tau <= g.on_time;
+    o.env[2 * blockIdx.y] = on ? 1.0 : 0.0;
+    o.env[2 * blockIdx.y + 1] = on ? g.pamp * burst_env(g, tau) : 0.0;
+  }
+  if (e >= elems) return;
+  double sn, cs;
+  sincos(g.omega * t + g.elem_phase[e], &sn, &cs);
+  o.sn[(size_t)blockIdx.y * elems + e] = sn;
+  o.cs[(size_t)blockIdx.y * elems + e] = cs;
+}
+
+// Source cell c (frame index cells[c], element elem[c]) at the step whose factors
+// these are: d p'_x / d amp_e and d p'_x / d phase_e times the adjoint of p'_x, summed
 // over the steps per cell; the cell's adjoints then end (the forced values do
 // not depend on the state).
 __global__ void adj3_source(const __grid_constant__ Grid3 g, const Adj3 a, const long* cells, const int* elem, int n,
-                            double t, double* gA, double* gP) {
+                            const SourceFactors t, double* gA, double* gP) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const long q = cells[c];
@@ -1063,78 +1086,115 @@ __global__ void adj3_source(const __grid_constant__ Grid3 g, const Adj3 a, const
   a.MX[q] = 0.0;
   a.MY[q] = 0.0;
   a.MZ[q] = 0.0;
-  if (!(t > 0.0)) return;
-  const double tau = fmod(t, g.period);
-  if (!(tau <= g.on_time)) return;
+  if (t.env[0] == 0.0) return;
+  const double env = t.env[1];
   const int e = elem[c];
-  double sn, cs;
-  sincos(g.omega * t + g.elem_phase[e], &sn, &cs);
-  const double env = g.pamp * burst_env(g, tau);
-  gA[c] += m * env * sn;
-  gP[c] += m * env * g.elem_amp[e] * cs;
-}
-
-// The pressure update's transpose at one face (computed faces: vx for i in
-// [0, X] with j, k interior; vy for j in [0, Y]; vz for k in [0, Z]).
-__device__ __forceinline__ double adj3_lxt(const Grid3& g, const Adj3& a, int i, int j, int k) {
-  const Frame3& f = g.f;
-  const long q = f.idx(i, j, k);
-  return a.LX[q] + (-g.s3p) * g.rdx * (g.pbx[i] * a.MX[q] - g.pbx[i + 1] * a.MX[f.idx(i + 1, j, k)]);
-}
-__device__ __forceinline__ double adj3_lyt(const Grid3& g, const Adj3& a, int i, int j, int k) {
-  const Frame3& f = g.f;
-  const long q = f.idx(i, j, k);
-  return a.LY[q] + (-g.s3p) * g.rdy * (g.pby[j] * a.MY[q] - g.pby[j + 1] * a.MY[f.idx(i, j + 1, k)]);
-}
-__device__ __forceinline__ double adj3_lzt(const Grid3& g, const Adj3& a, int i, int j, int k) {
-  const Frame3& f = g.f;
-  const long q = f.idx(i, j, k);
-  return a.LZ[q] + (-g.s3p) * g.rdz * (g.pbz[k] * a.MZ[q] - g.pbz[k + 1] * a.MZ[f.idx(i, j, k + 1)]);
+  gA[c] += m * env * t.sn[e];
+  gP[c] += m * env * g.elem_amp[e] * t.cs[e];
 }
 
 // One reverse step after adj3_source, from `in` into `out`; p0 (the focal
-// pressures of the step before, or null) adds that step's objective term.
-// Blocks of 32 x 8 cells of one plane (blockIdx.z); each interior cell writes
-// its east, north and top faces, the first column, row and plane also the
-// 0 faces.
-__global__ void adj3_step(const __grid_constant__ Grid3 g, const Adj3 in, const Adj3 out, const Box3 b,
-                          const double* __restrict__ p0, double two_dt) {
+// pressures of the step before, or null) adds that step's objective term.  Warps of 64
+// columns, two per lane, march along z as in fdtd3; the value of the face below is that
+// of the top face one plane down.  Every lane forms the transposed values
+// L + s3p rd (pb_b M_b - pb_a M_a) of its faces (computed faces: vx for i in [0, X] with j,
+// k interior; vy for j in [0, Y]; vz for k in [0, Z]); the first column, row and plane also
+// write the 0 faces.  Bound by the latency of the loads at 16 warps per SM: 141 x 125 x 133
+// takes 45.9 us (96 bytes per cell: 4.9 TB/s), 56 with one cell per thread.
+__global__ void __launch_bounds__(32 * kRows3, 2) adj3_march(const __grid_constant__ Grid3 g, const Adj3 in,
+                                                             const Adj3 out, const Box3 b,
+                                                             const double* __restrict__ p0, double two_dt, int planes) {
   const Frame3& f = g.f;
-  const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y * blockDim.y + threadIdx.y,
-            k = 1 + blockIdx.z;
-  if (i > f.X || j > f.Y || k > f.Z) return;
-  const long q = f.idx(i, j, k);
-  const double xe = adj3_lxt(g, in, i, j, k), xw = adj3_lxt(g, in, i - 1, j, k);
-  const double yn = adj3_lyt(g, in, i, j, k), ys = adj3_lyt(g, in, i, j - 1, k);
-  const double zt = adj3_lzt(g, in, i, j, k), zb = adj3_lzt(g, in, i, j, k - 1);
-  const double lp0 = g.dt_rho * (g.rdx * (g.vbx[i + 1] * xe - g.vbx[i] * xw) +
-                                 g.rdy * (g.vby[j + 1] * yn - g.vby[j] * ys) +
-                                 g.rdz * (g.vbz[k + 1] * zt - g.vbz[k] * zb));
-  double mx = g.pax[i] * in.MX[q] + lp0;
-  double my = g.pay[j] * in.MY[q] + lp0;
-  double mz = g.paz[k] * in.MZ[q] + lp0;
-  if (p0) {
-    const int bi = i - b.i0, bj = j - b.j0, bk = k - b.k0;
-    if (bi >= 0 && bi < b.nx && bj >= 0 && bj < b.ny && bk >= 0 && bk < b.nz) {
-      const long t = bi + (long)b.nx * (bj + (long)b.ny * bk);
-      const double w = b.w[t];
-      if (w != 0.0) {
-        const double d = two_dt * w * p0[t];
-        mx += d;
-        my += d;
-        mz += d;
+  const int i = 1 + blockIdx.x * kCols3 + 2 * threadIdx.x, j = 1 + blockIdx.y * kRows3 + threadIdx.y;
+  const int k0 = 1 + blockIdx.z * planes, k1 = min(f.Z, k0 + planes - 1);
+  if (i > f.X || j > f.Y) return;
+  const bool two = i + 1 <= f.X;
+  const unsigned pitch = (unsigned)f.pitch, plane = (unsigned)(f.Y + 4) * pitch;
+  auto get2 = [](const double* p, unsigned q) { return *reinterpret_cast<const double2*>(p + q); };
+  const double sx = -g.s3p * g.rdx, sy = -g.s3p * g.rdy, sz = -g.s3p * g.rdz;
+  // Lt of the face between cells a and b.
+  auto lt = [](double L, double s, double pa, double ma, double pb, double mb) -> double {
+    return fma(s, fma(pa, ma, -__dmul_rn(pb, mb)), L);
+  };
+  double pbx[4], vbx[3], ax[3], pax[2];
+#pragma unroll
+  for (int c = 0; c < 4; c++) pbx[c] = g.pbx[min(i - 1 + c, f.X + 1)];
+#pragma unroll
+  for (int c = 0; c < 3; c++) vbx[c] = g.vbx[i + c], ax[c] = g.vax[i + c] * vbx[c];
+  pax[0] = g.pax[i], pax[1] = g.pax[i + 1];
+  const double pbs = g.pby[j - 1], pbj = g.pby[j], pbn = g.pby[j + 1], pay = g.pay[j];
+  const double vbs = g.vby[j], vbn = g.vby[j + 1], ayn = g.vay[j + 1] * vbn, ays = g.vay[j] * vbs;
+  unsigned q = ((unsigned)(k0 + 1) * (unsigned)(f.Y + 4) + (unsigned)(j + 1)) * pitch + (unsigned)(i + 1);
+  double2 mz = get2(in.MZ, q);
+  double zb[2];
+  {
+    const double2 l = get2(in.LZ, q - plane), m = get2(in.MZ, q - plane);
+    const double pa = g.pbz[k0 - 1], pb = g.pbz[k0];
+    zb[0] = lt(l.x, sz, pa, m.x, pb, mz.x);
+    zb[1] = lt(l.y, sz, pa, m.y, pb, mz.y);
+  }
+#pragma unroll 1
+  for (int k = k0; k <= k1; k++, q += plane) {
+    const double2 lx = get2(in.LX, q), ly = get2(in.LY, q), ls = get2(in.LY, q - pitch), lz = get2(in.LZ, q);
+    const double2 mx = get2(in.MX, q), my = get2(in.MY, q), ms = get2(in.MY, q - pitch), mn = get2(in.MY, q + pitch);
+    const double2 mu = get2(in.MZ, q + plane);
+    const double lw = in.LX[q - 1], mw = in.MX[q - 1], me = in.MX[q + 2];
+    const double m4[4] = {mw, mx.x, mx.y, me}, l3[3] = {lw, lx.x, lx.y};
+    double xt[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) xt[c] = lt(l3[c], sx, pbx[c], m4[c], pbx[c + 1], m4[c + 1]);
+    const double yn[2] = {lt(ly.x, sy, pbj, my.x, pbn, mn.x), lt(ly.y, sy, pbj, my.y, pbn, mn.y)};
+    const double ys[2] = {lt(ls.x, sy, pbs, ms.x, pbj, my.x), lt(ls.y, sy, pbs, ms.y, pbj, my.y)};
+    const double pbk = g.pbz[k], pbu = g.pbz[k + 1], vbt = g.vbz[k + 1], vbb = g.vbz[k];
+    const double zt[2] = {lt(lz.x, sz, pbk, mz.x, pbu, mu.x), lt(lz.y, sz, pbk, mz.y, pbu, mu.y)};
+    const double azt = g.vaz[k + 1] * vbt, paz = g.paz[k];
+    const double m3[2][3] = {{mx.x, my.x, mz.x}, {mx.y, my.y, mz.y}};
+    double nm[3][2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      const double dx = fma(vbx[c + 1], xt[c + 1], -__dmul_rn(vbx[c], xt[c]));
+      const double dy = fma(vbn, yn[c], -__dmul_rn(vbs, ys[c]));
+      const double dz = fma(vbt, zt[c], -__dmul_rn(vbb, zb[c]));
+      const double lp0 = __dmul_rn(g.dt_rho, fma(g.rdz, dz, fma(g.rdx, dx, __dmul_rn(g.rdy, dy))));
+      nm[0][c] = fma(pax[c], m3[c][0], lp0);
+      nm[1][c] = fma(pay, m3[c][1], lp0);
+      nm[2][c] = fma(paz, m3[c][2], lp0);
+      if (p0) {
+        const int bi = i + c - b.i0, bj = j - b.j0, bk = k - b.k0;
+        if (bi >= 0 && bi < b.nx && bj >= 0 && bj < b.ny && bk >= 0 && bk < b.nz) {
+          const long t = bi + (long)b.nx * (bj + (long)b.ny * bk);
+          const double w = b.w[t];
+          if (w != 0.0) {
+            const double d = __dmul_rn(two_dt * w, p0[t]);
+            nm[0][c] += d;
+            nm[1][c] += d;
+            nm[2][c] += d;
+          }
+        }
       }
     }
+    auto put = [&](double* p, unsigned r, double v, double w) {
+      if (two)
+        *reinterpret_cast<double2*>(p + r) = make_double2(v, w);
+      else
+        p[r] = v;
+    };
+    put(out.MX, q, nm[0][0], nm[0][1]);
+    put(out.MY, q, nm[1][0], nm[1][1]);
+    put(out.MZ, q, nm[2][0], nm[2][1]);
+    put(out.LX, q, xt[1] * ax[1], xt[2] * ax[2]);
+    put(out.LY, q, yn[0] * ayn, yn[1] * ayn);
+    put(out.LZ, q, zt[0] * azt, zt[1] * azt);
+    if (i == 1) out.LX[q - 1] = xt[0] * ax[0];
+    if (j == 1) put(out.LY, q - pitch, ys[0] * ays, ys[1] * ays);
+    if (k == 1) {
+      const double az0 = g.vaz[1] * g.vbz[1];
+      put(out.LZ, q - plane, zb[0] * az0, zb[1] * az0);
+    }
+    zb[0] = zt[0];
+    zb[1] = zt[1];
+    mz = mu;
   }
-  out.MX[q] = mx;
-  out.MY[q] = my;
-  out.MZ[q] = mz;
-  out.LX[q] = xe * (g.vax[i + 1] * g.vbx[i + 1]);
-  out.LY[q] = yn * (g.vay[j + 1] * g.vby[j + 1]);
-  out.LZ[q] = zt * (g.vaz[k + 1] * g.vbz[k + 1]);
-  if (i == 1) out.LX[f.idx(0, j, k)] = xw * (g.vax[1] * g.vbx[1]);
-  if (j == 1) out.LY[f.idx(i, 0, k)] = ys * (g.vay[1] * g.vby[1]);
-  if (k == 1) out.LZ[f.idx(i, j, 0)] = zb * (g.vaz[1] * g.vbz[1]);
 }
 
 }  // namespace d3
@@ -1267,6 +1327,14 @@ struct Sim3Impl {
 
   crp_status create(const crp_config& c, const crp_bubbles_in* bin, void* user_stream);
   crp_status step_once();
+  // Planes per chunk of the marching passes: up to 16 (256^3: 398 us, 425 with 32, 402
+  // with 8), fewer where that would leave less than two waves of the 296 blocks that the
+  // GPU holds; blocks: of one chunk.
+  int march3_planes(long blocks) const {
+    int planes = d3::kPlanes3;
+    while (planes > 2 && blocks * ((g.f.Z + planes - 1) / planes) < 4 * 148) planes /= 2;
+    return planes;
+  }
   // Steps without bubbles, queued back to back: `left` more follow in this call.
   // Nothing the host decides depends on their scalars; finish_plain reads those of the
   // last step (a non-finite pressure stays non-finite in the linear step).
@@ -1702,10 +1770,7 @@ crp_status Sim3Impl::launch_fdtd(const double* elem) {
   a.coupling = (int)coupling + 1;
   a.elem_p = elem;
   const int sx = (g.f.X + d3::kCols3 - 1) / d3::kCols3, sy = (g.f.Y + d3::kRows3 - 1) / d3::kRows3;
-  // Planes per chunk: up to 16 (256^3: 398 us, 425 with 32, 402 with 8), fewer where that
-  // would leave less than two waves of the 296 blocks that the GPU holds.
-  int planes = d3::kPlanes3;
-  while (planes > 2 && (long)sx * sy * ((g.f.Z + planes - 1) / planes) < 4 * 148) planes /= 2;
+  const int planes = march3_planes(sx * sy);
   const dim3 block(32, d3::kRows3), grid(sx, sy, (g.f.Z + planes - 1) / planes);
   int u[6], w[6];
   box_union(w, supp[0], supp[1]);
@@ -2001,7 +2066,8 @@ crp_status Sim3Impl::adjoint(const crp_objective* obj, double* J, double* grad_a
   // Two sets of six adjoint frames, per-source-cell gradients, weights,
   // history, objective per step; then the source cells' frame indices and
   // elements.
-  const size_t n_doubles = 12 * cells + 2 * (size_t)ns1 + box_n + hist_n + (size_t)N;
+  const size_t n_fac = d3::kElemBatch * (2 + 2 * (size_t)elem_n);
+  const size_t n_doubles = 12 * cells + 2 * (size_t)ns1 + box_n + hist_n + (size_t)N + n_fac;
   const size_t bytes = n_doubles * sizeof(double) + (size_t)ns1 * (sizeof(long) + sizeof(int));
   // The workspace is kept for the next call and released with the simulation.
   if (adj_ws_bytes < bytes) {
@@ -2034,6 +2100,9 @@ crp_status Sim3Impl::adjoint(const crp_objective* obj, double* J, double* grad_a
   double* d_w = gP + ns1;
   double* hist = d_w + box_n;
   double* d_Jn = hist + hist_n;
+  double* d_env = d_Jn + N;
+  double* d_sn = d_env + 2 * d3::kElemBatch;
+  const d3::SourceFactors fac{d_env, d_sn, d_sn + (size_t)d3::kElemBatch * elem_n};
   long* d_cells = reinterpret_cast<long*>(base + n_doubles);
   int* d_el = reinterpret_cast<int*>(d_cells + ns1);
   C3(cudaMemsetAsync(buf, 0, n_doubles * sizeof(double), stream));
@@ -2074,7 +2143,9 @@ crp_status Sim3Impl::adjoint(const crp_objective* obj, double* J, double* grad_a
   for (int n = 0; n < N; n++) Jsum += Jn[n];
   if (J) *J = g.dt * Jsum;
   // Reverse sweep: reverse step n reads frame set s and writes set s ^ 1.
-  const dim3 sblk(32, 8), sgrid((f.X + 31) / 32, (f.Y + 7) / 8, f.Z);
+  const int sx = (f.X + d3::kCols3 - 1) / d3::kCols3, sy = (f.Y + d3::kRows3 - 1) / d3::kRows3;
+  const int planes = march3_planes(sx * sy);
+  const dim3 sblk(32, d3::kRows3), sgrid(sx, sy, (f.Z + planes - 1) / planes);
   const int sb = (ns + 255) / 256;
   const double two_dt = 2.0 * g.dt;
   d3::adj3_force<<<rb, 256, 0, stream>>>(f, fr[0], box, hist + (size_t)(N - 1) * box_n, two_dt);
@@ -2082,11 +2153,21 @@ crp_status Sim3Impl::adjoint(const crp_objective* obj, double* J, double* grad_a
   int s = 0;
   for (int n = N; n >= 1; n--, s ^= 1) {
     if (ns > 0) {
-      d3::adj3_source<<<sb, 256, 0, stream>>>(g, fr[s], d_cells, d_el, ns, times[n], gA, gP);
+      const int q = (N - n) % d3::kElemBatch;
+      if (q == 0) {
+        d3::ElemTimes et{};
+        const int m = std::min(n, d3::kElemBatch);
+        for (int r = 0; r < m; r++) et.t[r] = times[n - r];
+        const dim3 grid(elem_n / d3::kBeginThreads3 + 1, m);
+        d3::adj3_factors<<<grid, d3::kBeginThreads3, 0, stream>>>(g, et, elem_n, fac);
+        launches++;
+      }
+      const d3::SourceFactors t{fac.env + 2 * q, fac.sn + (size_t)q * elem_n, fac.cs + (size_t)q * elem_n};
+      d3::adj3_source<<<sb, 256, 0, stream>>>(g, fr[s], d_cells, d_el, ns, t, gA, gP);
       launches++;
     }
     const double* p0 = n >= 2 ? hist + (size_t)(n - 2) * box_n : nullptr;
-    d3::adj3_step<<<sgrid, sblk, 0, stream>>>(g, fr[s], fr[s ^ 1], box, p0, two_dt);
+    d3::adj3_march<<<sgrid, sblk, 0, stream>>>(g, fr[s], fr[s ^ 1], box, p0, two_dt, planes);
     C3(cudaGetLastError());
     launches++;
   }
