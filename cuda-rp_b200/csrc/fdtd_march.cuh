@@ -32,6 +32,13 @@ constexpr int kMarchCols = 64;  // columns of a warp
 // 40.1, 5 blocks (96 registers, more spilled) 29.4 and 43.1, 3 blocks 29.0 and 43.4.
 constexpr int kMarchMinBlocks = 4;
 
+// Where the pass leaves p0 of the previous step on the cells [i0, i0 + w) x [j0, j0 + h)
+// (the focal history of the adjoint: 3 us per step less than a launch of its own).
+struct FocalRecord {
+  int i0, j0, w, h;
+  double* out;  // null: nowhere
+};
+
 template <typename P>
 struct MarchRow {
   double2 x, y;           // px, py of the lane's two columns
@@ -42,9 +49,9 @@ struct MarchRow {
 // and any void fraction, of which it knows nothing; kEdges without void fraction;
 // kVoid for everything.  Lane columns i and i + 1 (i odd, i <= X), rows j0..j1.
 enum MarchForm { kPlain = 0, kEdges = 1, kVoid = 2 };
-template <typename P, int FORM>
-__device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, const FdtdArgs<P>& a, int i, int j0,
-                                                          int j1) {
+template <typename P, int FORM, bool REC>
+__device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, const FdtdArgs<P>& a,
+                                                          const FocalRecord& rec, int i, int j0, int j1) {
   constexpr bool GEN = FORM >= kEdges, VOID = FORM == kVoid;
   using G = typename P::G;
   const Frame& f = g.f;
@@ -188,6 +195,11 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
       vy2 = a.vy_old.get2(k + pitch);
       vxl = a.vx_old.get(k + pitch - 1);
     }
+    if (REC && (unsigned)(j - rec.j0) < (unsigned)rec.h) {
+#pragma unroll
+      for (int c = 0; c < 2; c++)
+        if ((unsigned)(i + c - rec.i0) < (unsigned)rec.w) rec.out[(unsigned)(j - rec.j0) * (unsigned)rec.w + (unsigned)(i + c - rec.i0)] = pc[c + 1];
+    }
     double pu[4], ru[4], fu[2], fgp[2], h[2] = {0.0, 0.0};
     pressures(up, j + 1, pu);
     if (GEN && j == Y) {  // p0 of the y1 ghost row: PML, or the mirror of row Y
@@ -274,9 +286,11 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
   return res;
 }
 
-template <typename P>
+// REC: with the record (only without bubbles).
+template <typename P, bool REC>
 __global__ void __launch_bounds__(32 * kMarchWarps, kMarchMinBlocks) fdtd_march(const __grid_constant__ GridParams g,
-                                                                  const FdtdArgs<P> a, int rows, int strips) {
+                                                                  const FdtdArgs<P> a, const FocalRecord rec, int rows,
+                                                                  int strips) {
   const int X = g.f.X, Y = g.f.Y;
   const int lane = threadIdx.x & 31;
   const int strip = blockIdx.x % strips, chunk = (blockIdx.x / strips) * kMarchWarps + (threadIdx.x >> 5);
@@ -298,12 +312,12 @@ __global__ void __launch_bounds__(32 * kMarchWarps, kMarchMinBlocks) fdtd_march(
                      (g.source_row >= j0 - 1 && g.source_row <= j1 + 1 && g.source_row > 0);
   unsigned long long res = 0ull;
   if (i <= X) {
-    if (fg)
-      res = march_chunk<P, kVoid>(g, a, i, j0, j1);
+    if (!REC && fg)
+      res = march_chunk<P, kVoid, false>(g, a, rec, i, j0, j1);
     else if (edges)
-      res = march_chunk<P, kEdges>(g, a, i, j0, j1);
+      res = march_chunk<P, kEdges, REC>(g, a, rec, i, j0, j1);
     else
-      res = march_chunk<P, kPlain>(g, a, i, j0, j1);
+      res = march_chunk<P, kPlain, REC>(g, a, rec, i, j0, j1);
   }
   // Warp maximum, one atomic per warp with a nonzero residual.
   for (int o = 16; o > 0; o >>= 1) res = max(res, __shfl_xor_sync(0xffffffffu, res, o));

@@ -2020,6 +2020,7 @@ struct Sim {
   // three launches, 26 with one).
   bool plain_ok() const { return hs.nb == 0 && !temperature_on && !prof.on && !debug_picard && stats.steps > 0; }
   int src_next = 0, src_n = 0;  // steps of the current batch used and evaluated
+  FocalRecord focal_rec{};      // what the next queued step records (adjoint)
   // One step, `left` more to follow in this call.
   crp_status queue_plain(int left) {
     if (fdtd_tma_on) {
@@ -2589,7 +2590,13 @@ struct Sim {
       const int strips = (gp.f.X + kMarchCols - 1) / kMarchCols, rows = march_rows(strips);
       const int chunks = (gp.f.Y + rows - 1) / rows;
       const int grid = strips * ((chunks + kMarchWarps - 1) / kMarchWarps);
-      e = launch(kClassFdtd, [&] { fdtd_march<P><<<grid, 32 * kMarchWarps, 0, stream>>>(gp, fa, rows, strips); });
+      const FocalRecord rec = focal_rec;
+      if (rec.out)
+        e = launch(kClassFdtd,
+                   [&] { fdtd_march<P, true><<<grid, 32 * kMarchWarps, 0, stream>>>(gp, fa, rec, rows, strips); });
+      else
+        e = launch(kClassFdtd,
+                   [&] { fdtd_march<P, false><<<grid, 32 * kMarchWarps, 0, stream>>>(gp, fa, rec, rows, strips); });
     }
     return e;
   }
@@ -3114,23 +3121,35 @@ crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, d
   times[0] = tstep;
   bool queued = false;  // steps queued by queue_plain, checked by finish_plain
   src_next = src_n = 0;
-  for (int n = 1; n <= N; n++) {
-    const bool plain = plain_ok();
-    const crp_status st = plain ? queue_plain(N - n) : step_once();
-    if (st != CRP_OK) return st;
-    queued = queued || plain;
-    double* out = hist + (size_t)(n - 1) * cells_box;
-    cudaError_t e;
+  // p0 after a step is recorded by the next step's pass where that one is queued, else
+  // by a launch of its own.
+  double* due = nullptr;
+  auto record = [&]() -> cudaError_t {
+    double* out = due;
+    due = nullptr;
     if (mixed) {
       const F32c a = view<F32c>(px[cur_p]), b = view<F32c>(py[cur_p]);
-      e = launch(kClassOther, [&] { adj_record<F32c><<<rb, 256, 0, stream>>>(gp, a, b, box, out); });
-    } else {
-      const F64 a = view<F64>(px[cur_p]), b = view<F64>(py[cur_p]);
-      e = launch(kClassOther, [&] { adj_record<F64><<<rb, 256, 0, stream>>>(gp, a, b, box, out); });
+      return launch(kClassOther, [&] { adj_record<F32c><<<rb, 256, 0, stream>>>(gp, a, b, box, out); });
     }
-    CRP_CUDA(e);
+    const F64 a = view<F64>(px[cur_p]), b = view<F64>(py[cur_p]);
+    return launch(kClassOther, [&] { adj_record<F64><<<rb, 256, 0, stream>>>(gp, a, b, box, out); });
+  };
+  for (int n = 1; n <= N; n++) {
+    const bool plain = plain_ok();
+    if (due && plain && !fdtd_tma_on) {
+      focal_rec = FocalRecord{bi0, bj0, bw, bh, due};
+      due = nullptr;
+    } else if (due) {
+      CRP_CUDA(record());
+    }
+    const crp_status st = plain ? queue_plain(N - n) : step_once();
+    focal_rec = FocalRecord{};
+    if (st != CRP_OK) return st;
+    queued = queued || plain;
+    due = hist + (size_t)(n - 1) * cells_box;
     times[n] = tstep;
   }
+  CRP_CUDA(record());
   if (queued) {
     const crp_status st = finish_plain();
     if (st != CRP_OK) return st;
