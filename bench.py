@@ -73,12 +73,12 @@ WORKLOADS = {
     "cart3d_384": os.path.join(PKG, "configs", "cart3d_384.conf"),
     "cart3d_256": os.path.join(PKG, "configs", "cart3d_256.conf"),
 }
-# Compulsory HBM traffic of the fused FDTD pass per cell: FP64
-# reads px, py, vx, vy, f_g, f_gn, f_gm and writes px, py, vx, vy, predicted f_g;
-# mixed stores each velocity/pressure value as two FP32 words and f_g as FP32.
-BYTES_PER_CELL = {"fp64": 96, "mixed": 80}
-# 3-D: vz and pz besides, each read and written.
-BYTES_PER_CELL_3D = {"fp64": 128, "mixed": 112}
+# Compulsory HBM traffic of the fused FDTD pass per cell: px, py, vx, vy read and
+# written, 8 bytes each in both precisions (mixed stores a value as two FP32 words).
+# Cells where the void fraction can be nonzero move 32 (mixed 16) bytes more, not counted.
+BYTES_PER_CELL = {"fp64": 64, "mixed": 64}
+# 3-D: vz and pz besides.
+BYTES_PER_CELL_3D = {"fp64": 96, "mixed": 96}
 
 
 def is3d(cfg):
@@ -709,7 +709,7 @@ def run_ours(args, rank, world, dist):
         focal = guarded(compare_at, {p: r["sim"] for p, r in runs.items()}, cfg)
     hbm, kind = peaks()
     bpc = (BYTES_PER_CELL_3D if is3d(cfg) else BYTES_PER_CELL)[primary]
-    kernel = "fdtd3" if is3d(cfg) else "fdtd_strip"
+    kernel = "fdtd3" if is3d(cfg) else "fdtd_march"
     achieved = bpc * cells / (fdtd_ms * 1e-3) / 1e9 if n_fdtd else None
     result = None
     if rank == 0:

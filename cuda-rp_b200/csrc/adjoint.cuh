@@ -25,7 +25,7 @@
 // so the pass carries no transcendental code.  Per cell and step it reads 4 doubles
 // (L_x, L_y, M_x, M_y; the neighbours' values come through L1/L2) and writes 4: 64 bytes.
 // Bound by the latency of the loads at 16 warps per SM: 600 x 701 takes 11.6 us cold
-// (27 MB: 2.3 TB/s).  A call of 200 steps there took 8.2 ms with one cell per
+// (27 MB: 2.3 TB/s).  A call of 300 steps there took 8.2 ms with one cell per
 // thread, each reading the coefficients of its row and column again and evaluating
 // the source's derivatives where the source row lies, 7.5 with this pass, and 6.4 since the
 // FDTD pass records the focal pressures.

@@ -134,7 +134,7 @@ struct Fdtd3Args {
 // Bound by the latency of its loads at 16 warps per SM (128 registers); DRAM traffic is
 // 1.14 times the 96 bytes per cell.  256^3 with a small cloud 366 us (4.4 TB/s of the 96
 // bytes; 718 before, with each thread's inputs staged through shared memory and two
-// barriers per plane), 141 x 125 x 133 without bubbles 70 us (155).
+// barriers per plane), 141 x 125 x 133 without bubbles 61 us (155).
 constexpr int kRows3 = 8;   // warps per block
 constexpr int kCols3 = 64;  // columns per warp
 constexpr int kPlanes3 = 16;  // planes per chunk, at most

@@ -416,8 +416,9 @@ void crp_state_free(crp_state* state);
 
 /* Launch shapes (no reference counterpart), chosen by crp_batch_tune or set
  * directly; results are bit for bit the same under every setting.
- * fdtd_rows: rows per chunk of the 2-D FDTD strip kernel, 4, 8 (default) or 16
- * (the 3-D path accepts the value and ignores it).  rp_blocks: blocks of the
+ * fdtd_rows: 4, 8 (default) or 16: a warp of the 2-D FDTD pass marches up half as
+ * many rows, or fewer where the grid would leave the GPU idle (the 3-D path accepts
+ * the value and ignores it).  rp_blocks: blocks of the
  * persistent radius kernel (0, the default: one lane per bubble up to the
  * occupancy limit, rp_blocks_max, which crp_get_tuning reports; larger
  * values are clamped to it). */
