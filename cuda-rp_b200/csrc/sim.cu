@@ -22,6 +22,7 @@
 //                  void fraction can be nonzero
 // Buffers rotate instead of being copied: velocity and pressure ping-pong, the
 // void-fraction history is a three-buffer ring.
+#include <climits>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -181,7 +182,6 @@ __device__ __noinline__ double source_row_pressure(const GridParams& g, double x
   return sv;
 }
 
-constexpr long kMarchWarpsWanted = 148 * 12;  // of the 148 x 16 the GPU holds
 constexpr int kMarchRows = 8;  // default of the tuned rows (crp_set_tuning)
 
 }  // namespace crp
@@ -2532,14 +2532,22 @@ struct Sim {
     return fail(CRP_ERR_INVALID, "unknown field");
   }
 
-  // Rows per chunk of the FDTD pass: half the tuned number, fewer where that would
-  // leave the GPU short of warps (kMarchWarpsWanted).  Measured with 4 and 8 rows:
-  // 1001 x 1531 without bubbles 26.0 and 27.5 us, 1024 x 2048 with bubbles 40.1 and 46.6
-  // (the few chunks with void fraction, the slowest, end last).
+  // Rows per chunk of the marching passes: of the numbers up to half the tuned one, that
+  // whose blocks take the least time in full waves of the 4 per SM that the GPU holds,
+  // a chunk's start counted as two rows.  Per FDTD pass with 2, 3, 4, 6 and 8 rows (us, the
+  // rule's choice in brackets): 600 x 701 12.8, [11.1], 12.7, 14.8, 16.1; 1001 x 1531 29.0,
+  // 27.0, [25.9], 26.1, 27.6; 1024 x 2048 with bubbles 43.7, 39.6, [40.7], 41.1, 47.0;
+  // 256 x 512 takes 11.7 with [1] and 13.0 with 2.
   int march_rows(int strips) const {
-    int rows = strip_rows / 2;
-    while (rows > 1 && (long)strips * ((gp.f.Y + rows - 1) / rows) < kMarchWarpsWanted) rows >>= 1;
-    return rows;
+    const long slots = 148 * kMarchMinBlocks;
+    int best = 1;
+    long least = LONG_MAX;
+    for (int r = std::max(1, strip_rows / 2); r >= 1; r--) {
+      const long chunks = (gp.f.Y + r - 1) / r, blocks = strips * ((chunks + kMarchWarps - 1) / kMarchWarps);
+      const long t = (blocks + slots - 1) / slots * (r + 2);
+      if (t < least) least = t, best = r;
+    }
+    return best;
   }
 
   // Per-precision launches.
