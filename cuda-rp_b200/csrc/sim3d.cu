@@ -93,10 +93,12 @@ __device__ __forceinline__ double void_half3(const Grid3& g, double fg, double f
 // Tiles of 32 x 8 x 8 cells (ghost cells included) and the last coupling in which
 // bubbles touched each (mark_tiles).  Couplings are counted by the steps whose Picard
 // loop ran.  A step's void fraction is nonzero at most where bubbles touched it in that
-// coupling, or, without one, where it was in the three steps before; so the f_g of a
-// step and of the two before it reach back six couplings at most, and a tile not
-// touched since holds zeros only.
-constexpr int kTile3X = 32, kTile3Y = 8, kTile3Z = 8, kTileLife = 6;
+// coupling, or, without one, where it was in the three steps before.  Steps without a
+// coupling can so hand an old coupling's void fraction on for as long as one of them
+// falls into every three steps; the host keeps the oldest coupling that each of the last
+// three steps reaches back to, and a tile not touched since the oldest of them holds
+// zeros only.
+constexpr int kTile3X = 32, kTile3Y = 8, kTile3Z = 8;
 struct Tiles3 {
   int nx, ny, nz;
   int* last;  // coupling index of the last touch (very negative: never)
@@ -115,7 +117,7 @@ struct Fdtd3Args {
   int bubbles;
   int supp[3][6];
   Tiles3 tiles;
-  int coupling;          // index of the next coupling
+  int oldest;            // coupling that the void fraction reaches back to
   const double* elem_p;  // pressure of every source element at the end of the step
   unsigned long long* residual;
 };
@@ -363,7 +365,7 @@ __global__ void __launch_bounds__(32 * kRows3, 2) fdtd3(const __grid_constant__ 
       bool live = false;
       for (int t = lane; t < nx * ny * nz; t += 32) {
         const int last = a.tiles.last[a.tiles.at(x0 + t % nx, y0 + t / nx % ny, z0 + t / (nx * ny))];
-        live = live || a.coupling - last <= kTileLife;
+        live = live || last >= a.oldest;
       }
       fg = __any_sync(0xffffffffu, live);
     }
@@ -823,7 +825,7 @@ struct TileRange {
   int lo[3], n[3];
 };
 __global__ void __launch_bounds__(256) mark_tiles(const Frame3 f, const int* __restrict__ start, Tiles3 t,
-                                                  TileRange r, int coupling, int* __restrict__ n_tiles) {
+                                                  TileRange r, int coupling, int oldest, int* __restrict__ n_tiles) {
   const int q = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (q >= r.n[0] * r.n[1] * r.n[2]) return;
   const int tile = t.at(r.lo[0] + q % r.n[0], r.lo[1] + q / r.n[0] % r.n[1], r.lo[2] + q / (r.n[0] * r.n[1]));
@@ -840,7 +842,7 @@ __global__ void __launch_bounds__(256) mark_tiles(const Frame3 f, const int* __r
   if (lane != 0) return;
   int last = t.last[tile];
   if (some) t.last[tile] = last = coupling;
-  if (coupling - last <= kTileLife) t.list[atomicAdd(n_tiles, 1)] = tile;
+  if (last >= oldest) t.list[atomicAdd(n_tiles, 1)] = tile;
 }
 
 // Per cell of the active tiles: the void fraction from the eight bins whose bubbles
@@ -1368,6 +1370,8 @@ struct Sim3Impl {
   crp_status launch_couple(bool pressure);
   d3::Tiles3 tiles{};
   int64_t coupling = 0;  // couplings so far: steps whose Picard loop ran
+  int64_t reach[3]{};    // oldest coupling in the void fraction of the last three steps (Tiles3)
+  int64_t oldest() const { return std::min(reach[0], std::min(reach[1], reach[2])); }
   // The active tiles of the next couplings of this step, from the current bins;
   // now: the bubbles' box.
   crp_status mark_tiles(const int now[6]);
@@ -1769,7 +1773,7 @@ crp_status Sim3Impl::launch_fdtd(const double* elem) {
   a.bubbles = bub.n > 0 ? 1 : 0;
   std::memcpy(a.supp, supp, sizeof(a.supp));
   a.tiles = tiles;
-  a.coupling = (int)coupling + 1;
+  a.oldest = (int)oldest();
   a.elem_p = elem;
   const int sx = (g.f.X + d3::kCols3 - 1) / d3::kCols3, sy = (g.f.Y + d3::kRows3 - 1) / d3::kRows3;
   const int planes = march3_planes(sx * sy);
@@ -1845,7 +1849,7 @@ crp_status Sim3Impl::mark_tiles(const int now[6]) {
     r.n[q] = box[q + 3] / size[q] - r.lo[q] + 1;
   }
   d3::mark_tiles<<<(r.n[0] * r.n[1] * r.n[2] + 7) / 8, 256, 0, stream>>>(g.f, bin_start, tiles, r, (int)coupling,
-                                                                          &d_sc->tiles);
+                                                                          (int)oldest(), &d_sc->tiles);
   C3(cudaGetLastError());
   launches++;
   return CRP_OK;
@@ -2008,6 +2012,10 @@ crp_status Sim3Impl::step_once() {
   std::memcpy(supp[2], supp[1], sizeof(snow));
   std::memcpy(supp[1], supp[0], sizeof(snow));
   std::memcpy(supp[0], snow, sizeof(snow));
+  const int64_t back = loop > 0 ? coupling : oldest();
+  reach[2] = reach[1];
+  reach[1] = reach[0];
+  reach[0] = back;
   stats.steps++;
   stats.time = tstep;
   stats.picard_last = loop;
@@ -2329,7 +2337,7 @@ struct HostState3 {
   int cur_v, cur_p, fg_a, fg_b, fg_c, bins_stale;
   double tstep, tstepx, t_prev;
   int supp[3][6];
-  int64_t coupling;
+  int64_t coupling, reach[3];
   crp_stats stats;
   d3::Scalars3 hsc;
 };
@@ -2346,6 +2354,7 @@ crp_status sim3_save_state(Sim3Impl* s, void* blob, std::vector<unsigned char>& 
   h.stats = s->stats;
   h.hsc = *s->h_sc;
   h.coupling = s->coupling;
+  std::memcpy(h.reach, s->reach, sizeof(h.reach));
   host.resize(sizeof(HostState3));
   std::memcpy(host.data(), &h, sizeof(HostState3));
   return CRP_OK;
@@ -2362,6 +2371,7 @@ crp_status sim3_load_state(Sim3Impl* s, const void* blob, const std::vector<unsi
   s->tstep = h.tstep, s->tstepx = h.tstepx, s->t_prev = h.t_prev;
   std::memcpy(s->supp, h.supp, sizeof(h.supp));
   s->coupling = h.coupling;
+  std::memcpy(s->reach, h.reach, sizeof(s->reach));
   const crp_stats keep = s->stats;
   s->stats = h.stats;
   s->stats.kernel_launches = keep.kernel_launches;
