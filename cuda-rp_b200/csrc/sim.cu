@@ -2091,7 +2091,7 @@ struct Sim {
       if (substep_prev > kLptMinSubsteps) CRP_CUDA(build_order());
       CRP_CUDA(launch(kClassOther,
                       [&] { picard_gate<<<1, 1, 0, stream>>>(d_scalars, gp.P_inf, picard_tol, hs.nb); }));
-      CRP_CUDA(mixed ? launch_rp<PrecMixed>() : launch_rp<PrecFP64>());
+      CRP_CUDA(mixed ? launch_rp<PrecMixed>(substep_prev) : launch_rp<PrecFP64>(substep_prev));
       CRP_CUDA(cudaEventSynchronize(ev));
     } else {
       CRP_CUDA(wait_stream());
@@ -2118,7 +2118,8 @@ struct Sim {
         loop++;
         if (!(first_queued && loop == 1)) {
           CRP_CUDA(launch(kClassOther, [&] { picard_begin<<<1, 1, 0, stream>>>(d_scalars, loop - 1); }));
-          CRP_CUDA(mixed ? launch_rp<PrecMixed>() : launch_rp<PrecFP64>());
+          const long long substeps = h_scalars->substep_max;
+          CRP_CUDA(mixed ? launch_rp<PrecMixed>(substeps) : launch_rp<PrecFP64>(substeps));
         }
         CRP_CUDA(launch_couple(true));
         st = read_scalars();
@@ -2343,7 +2344,7 @@ struct Sim {
     if (be == cudaSuccess) be = capture(body3, {}, sinks, [&] { return build_bins(); });
     if (be == cudaSuccess)
       be = capture(body4, {}, sinks, [&]() -> cudaError_t {
-        cudaError_t x = mixed ? launch_rp<PrecMixed>() : launch_rp<PrecFP64>();
+        cudaError_t x = mixed ? launch_rp<PrecMixed>(0) : launch_rp<PrecFP64>(0);
         if (x != cudaSuccess) return x;
         x = launch_couple(true);
         if (x != cudaSuccess) return x;
@@ -2751,7 +2752,6 @@ struct Sim {
 
   // The radius kernel of this simulation: rk45, or the reference scheme in the
   // form its temperature branch asks for (RadiusForm).
-  // A graph's launches cannot choose by the sub-steps so far; they take the quiet one.
   template <typename P>
   auto radius_kernel(bool tight) const {
     return cfg.ext_rp_scheme == CRP_RP_RK45 ? bubble_rk45<P>
@@ -2763,11 +2763,14 @@ struct Sim {
   cudaError_t radius_occupancy(int* per_sm, bool tight) const {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, radius_kernel<P>(tight), kRpThreads, 0);
   }
+  // substeps: the largest sub-step count that the host has read back so far (0 in a
+  // graph: its launches cannot choose by it and take the quiet instance).  A value, as
+  // the host's copy of the scalars may be in flight here.
   template <typename P>
-  cudaError_t launch_rp() {
+  cudaError_t launch_rp(long long substeps) {
     using S = typename P::S;
     const S pxc = view<S>(px[cur_p]), pyc = view<S>(py[cur_p]);
-    const bool tight = !capturing && h_scalars->substep_max >= kTightSubsteps;
+    const bool tight = substeps >= kTightSubsteps;
     const auto kernel = radius_kernel<P>(tight);
     const int grid = tight ? std::min(rp_grid, rp_grid_tight) : rp_grid;
     return launch(kClassRp, [&] {
