@@ -618,6 +618,8 @@ __device__ __forceinline__ double rroot4_pos(double x) {
 // The larger and the smaller of two numbers; b where a is NaN.
 __device__ __forceinline__ double larger(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ double smaller(double a, double b) { return a < b ? a : b; }
+// The smaller of two numbers; a where a is NaN.
+__device__ __forceinline__ double limited(double a, double b) { return a >= b ? b : a; }
 
 // Per-bubble constants of the FP64 radius solve: PG0 R0^3 and T0 / (PG0 R0^3)
 // (init_bub_params, src/bubble_CUDA.cu:666-670, PG0 = PL0 + 2 sigma / R0).

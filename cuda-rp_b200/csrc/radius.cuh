@@ -151,18 +151,20 @@ __device__ __forceinline__ void rp_substep_lean(const BubbleParams& b, RpState<T
     // The velocity and acceleration limits, 0.01 Rn / |d1R| and 0.1 Rn / sqrt(|acc|)
     // (:238-241): each quotient is formed only where it is the smaller step, decided
     // on the products (the squares for the second), so a quiet sub-step divides by
-    // neither.
+    // neither.  An infinite velocity or acceleration makes the quotient NaN (recip,
+    // rsqrt_pos) and with it the step and the remaining time: the solve stops as failed
+    // (rp_failed) where the reference takes steps of 0 up to the cap.
     const double net = fma(-(4.0 * b.mu * inv_Rn), d1n, fma(-2.0 * b.sig, inv_Rn, PGn - PL));
     const double acc = fma(net, b.inv_rho, -__dmul_rn(1.5 * d1n, d1n));
     dtp = smaller(1.01 * dtm, b.dt0);
     const double ad = fabs(d1n), aa = fabs(acc), lim = 0.1 * Rn;
     if (TIGHT) {
       const double tv = 0.01 * Rn * recip(ad), ta = lim * rsqrt_pos(aa);
-      dtp = ad > eps && 0.01 * Rn < dtp * ad ? smaller(tv, dtp) : dtp;
-      dtp = aa > eps && lim * lim < dtp * dtp * aa ? smaller(ta, dtp) : dtp;
+      dtp = ad > eps && 0.01 * Rn < dtp * ad ? limited(tv, dtp) : dtp;
+      dtp = aa > eps && lim * lim < dtp * dtp * aa ? limited(ta, dtp) : dtp;
     } else {
-      if (ad > eps && 0.01 * Rn < dtp * ad) dtp = smaller(0.01 * Rn * recip(ad), dtp);
-      if (aa > eps && lim * lim < dtp * dtp * aa) dtp = smaller(lim * rsqrt_pos(aa), dtp);
+      if (ad > eps && 0.01 * Rn < dtp * ad) dtp = limited(0.01 * Rn * recip(ad), dtp);
+      if (aa > eps && lim * lim < dtp * dtp * aa) dtp = limited(lim * rsqrt_pos(aa), dtp);
     }
     // q and 1 + q round as the reference's do: the rounding of 1 + q is the same at
     // every sub-step of a constant growth and acts on R as a small force, 1e-9 of a
@@ -225,6 +227,17 @@ __device__ __forceinline__ void rp_substep_lean(const BubbleParams& b, RpState<T
                         __dmul_rn(th.li, fma(PG, Rp3, -__dmul_rn(PGn, Rn3))));
   s.heat = fma(-(4.0 * b.pi * b.K0 * Rp * Rp), s.r.c.tpgr * hx * recip(wd), s.heat);
   s.vis = fma(16.0 * b.pi * b.mu * Rp * d1, d1 * dtp, s.vis);
+}
+
+// Whether a solve goes on, and whether one that does not was left unfinished: at the
+// cap, or with no step left (a remaining time of NaN).
+template <typename STATE>
+__device__ __forceinline__ bool rp_more(const BubbleParams& b, const STATE& s) {
+  return s.remain > 0.0 && s.count < b.step_cap;
+}
+template <typename STATE>
+__device__ __forceinline__ bool rp_failed(const STATE& s) {
+  return !(s.remain <= 0.0);
 }
 
 template <bool TIGHT, typename T, int FORM>

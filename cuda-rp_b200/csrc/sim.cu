@@ -680,10 +680,10 @@ __global__ void __launch_bounds__(kRpThreads, rp_min_blocks<P, TIGHT>()) bubble_
     }
     if (!__any_sync(0xffffffffu, n >= 0 || !drained)) break;
     if (n >= 0) {
-      if (s.remain > 0.0 && s.count < bp.step_cap) {
+      if (rp_more(bp, s)) {
         rp_substep_full<TIGHT>(bp, s);
       } else {
-        if (s.remain > 0.0) atomicOr(err, 1);
+        if (rp_failed(s)) atomicOr(err, 1);
         rp_end(g, bp, b, n, s);
         worst = max(worst, (long long)s.count);
         n = -1;

@@ -778,11 +778,11 @@ __global__ void __launch_bounds__(kRpThreads3, RK ? 1 : radius3_min_blocks<P, TI
       contrib3(g, bp, b, n, r.R);
       worst = max(worst, r.count);
     } else {
-      if (s.remain > 0.0 && s.count < bp.step_cap) {
+      if (rp_more(bp, s)) {
         rp_substep_full<TIGHT>(bp, s);
         continue;
       }
-      if (s.remain > 0.0) atomicOr(&sc->err, 1);
+      if (rp_failed(s)) atomicOr(&sc->err, 1);
       b.R_t[n] = s.Rt;
       b.R_p[n] = s.Rp;
       b.R_n[n] = s.Rn;
