@@ -87,6 +87,12 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
     if (i + 1 == X) q[3] = g.pml_x1 ? 0.0 : q[2];
   };
   auto rho_of = [&](double fa) -> double { return a.rho_const ? g.rho_inf : (1.0 - fa) * g.rho_inf; };
+  // dt / mean(rho) of a face, the same for both cells beside it and for every chunk:
+  // dt_rho, the plain forms' value, between densities of rho_inf (the quotient's last bit
+  // can differ from it).
+  auto face_factor = [&](double ra, double rb) -> double {
+    return ra == g.rho_inf && rb == g.rho_inf ? g.dt_rho : quotient(g.dt, (ra + rb) * 0.5);
+  };
   auto predict = [&](unsigned k) {  // a ghost cell's prediction
     a.fgC.put(k, G::stored(3.0 * a.fgA.get(k) - 3.0 * a.fgB.get(k) + a.fgC.get(k)));
   };
@@ -144,7 +150,7 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
     const double fa = g.vay[j0], fb = g.vby[j0];
 #pragma unroll
     for (int c = 0; c < 2; c++) {
-      const double q = VOID ? face_q(g, rb[c], rc[c + 1]) : g.dt_rho;
+      const double q = VOID ? face_factor(rb[c], rc[c + 1]) : g.dt_rho;
       vyd[c] = velocity_face_q(g, vo[c], pb[c + 1], pc[c + 1], q, fa, fb);
       if (GEN) {
         double pre = vyd[c];
@@ -221,11 +227,11 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
       a.fgC.put2(k, fgp[0], fgp[1]);  // the second is the ghost column where i = X
       if (i == 1) predict(k - 1);
       if (i + 1 == X) predict(k + 2);
-      // As face_q and void_rate_half; a quotient of equal densities rho_inf is dt_rho.
 #pragma unroll
-      for (int c = 0; c < 3; c++) qx[c] = quotient(g.dt, (rc[c] + rc[c + 1]) * 0.5);
-      qy[0] = quotient(g.dt, (rc[1] + ru[1]) * 0.5);
-      qy[1] = quotient(g.dt, (rc[2] + ru[2]) * 0.5);
+      for (int c = 0; c < 3; c++) qx[c] = face_factor(rc[c], rc[c + 1]);
+      qy[0] = face_factor(rc[1], ru[1]);
+      qy[1] = face_factor(rc[2], ru[2]);
+      // As void_rate_half.
 #pragma unroll
       for (int c = 0; c < 2; c++)
         h[c] = 0.5 * quotient(quotient(-(fgp[c] - fc[c]), g.dt), 1.0 - 0.5 * (fgp[c] + fc[c]));

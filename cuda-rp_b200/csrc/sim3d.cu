@@ -186,8 +186,11 @@ __device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const
   auto face = [&](double v, double p0a, double p0b, double q, double rh, double fa, double fb) -> double {
     return fma(v, fa, -__dmul_rn(q, (-p0a + p0b) * rh)) * fb;
   };
-  // dt / mean(rho) as face_q3 (a quotient of equal densities rho_inf is dt_rho).
-  auto slow = [&](double ra, double rb) -> double { return VOID ? quotient(g.dt, (ra + rb) * 0.5) : g.dt_rho; };
+  // dt / mean(rho) of a face, the same for every cell that forms it: dt_rho, the plain
+  // forms' value, between densities of rho_inf (the quotient's last bit can differ from it).
+  auto slow = [&](double ra, double rb) -> double {
+    return !VOID || (ra == g.rho_inf && rb == g.rho_inf) ? g.dt_rho : quotient(g.dt, (ra + rb) * 0.5);
+  };
   unsigned q = ((unsigned)k0 * (unsigned)(f.Y + 4) + (unsigned)(j + 1)) * pitch + (unsigned)(i + 1);  // plane k0 - 1
   const double vayn = g.vay[j + 1], vbyn = g.vby[j + 1], vays = g.vay[j], vbys = g.vby[j];
   const double pay = g.pay[j], pby = g.pby[j];
