@@ -32,7 +32,32 @@ __global__ void solve(const BubbleParams bp, int n, const double* pl, const doub
   out[2 * i + 1] = s.count;
 }
 
+// recip(b), quotient(a, b), rsqrt_pos(b), sqrt_pos(b), rroot4_pos(b), then the operators'
+// 1 / b, a / b, sqrt(b): rows of n values each.
+__global__ void helpers(int n, const double* a, const double* b, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double x = b[i];
+  const double v[8] = {recip(x),      quotient(a[i], x), rsqrt_pos(x), sqrt_pos(x),
+                       rroot4_pos(x), 1.0 / x,           a[i] / x,     sqrt(x)};
+  for (int q = 0; q < 8; q++) out[(size_t)q * n + i] = v[q];
+}
+
 }  // namespace
+
+extern "C" int units_helpers(int n, const double* a, const double* b, double* out) {
+  double* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, 10 * sizeof(double) * n);
+  if (e == cudaSuccess) e = cudaMemcpy(d, a, sizeof(double) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + n, b, sizeof(double) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    helpers<<<(n + 255) / 256, 256>>>(n, d, d + n, d + 2 * (size_t)n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, 8 * sizeof(double) * n, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return (int)e;
+}
 
 // form: 0 quiet lean, 1 lean for stiff launches, 2 lean of the mixed path, 3 with heat.
 extern "C" int units_solve(int form, int cap, int n, const double* pl, const double* v, int* out) {
