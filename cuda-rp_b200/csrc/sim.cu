@@ -941,14 +941,17 @@ __global__ void materialize_p0(const __grid_constant__ GridParams g, const S px,
 // read-back: the reads and writes cost microseconds and the host receives one
 // contiguous copy (mixed storage was converted value by value on the host: 5 ms for a
 // 1026 x 2050 field, a strided copy before it).  `scale`: the mixture density
-// (1 - f_g) rho_inf of a void-fraction value.
+// (1 - f_g) rho_inf of a void-fraction value.  Blocks stride over the rows: a grid may
+// have more of them than 8 per block of the largest launch.
 template <typename A>
 __global__ void dense_window(const Frame f, const A a, int ilo, int jlo, int w, int h, double rho_inf, int scale,
                              double* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= w || y >= h) return;
-  const double v = a.get(f.idx(ilo + x, jlo + y));
-  out[(long)y * w + x] = scale ? (1.0 - v) * rho_inf : v;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= w) return;
+  for (int y = blockIdx.y * blockDim.y + threadIdx.y; y < h; y += gridDim.y * blockDim.y) {
+    const double v = a.get(f.idx(ilo + x, jlo + y));
+    out[(long)y * w + x] = scale ? (1.0 - v) * rho_inf : v;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2185,7 +2188,7 @@ struct Sim {
   // double array.  kind: 0 FP64, 1 FP32 value + compensation, 2 FP32.
   crp_status copy_window(void* buf, int kind, int ilo, int ihi, int jlo, int jhi, double* host, bool density = false) {
     const int w = ihi - ilo + 1, h = jhi - jlo + 1;
-    const dim3 b(32, 8), grid((w + 31) / 32, (h + 7) / 8);
+    const dim3 b(32, 8), grid((w + 31) / 32, std::min((h + 7) / 8, 65535));
     const Frame f = gp.f;
     const double rho = gp.rho_inf;
     const int sc = density ? 1 : 0;
