@@ -91,14 +91,14 @@ __global__ void __launch_bounds__(64) source_derivative_rows(const __grid_consta
   out[(2 * (size_t)blockIdx.y + 1) * w + i] = dP;
 }
 
-constexpr int kAdjWarps = 4;
+constexpr int kAdjWarps = 4, kAdjMinBlocks = 4;
 
 // One reverse step: the transposes of the pressure update, the velocity update
 // and p0, from `in` into `out`; dA, dP: the source derivatives of the values that the
 // step read (null without elements).  p0 (the focal pressures of the step before, or
 // null for the first step) adds that step's objective term.
-__global__ void __launch_bounds__(32 * kAdjWarps, 4) adj_march(const __grid_constant__ GridParams g, const AdjFrames in,
-                                                               const AdjFrames out, const AdjGrad gr,
+__global__ void __launch_bounds__(32 * kAdjWarps, kAdjMinBlocks) adj_march(const __grid_constant__ GridParams g,
+                                                               const AdjFrames in, const AdjFrames out, const AdjGrad gr,
                                                                const double* __restrict__ dA,
                                                                const double* __restrict__ dP, const FocalBox b,
                                                                const double* __restrict__ p0, int rows, int strips) {

@@ -39,6 +39,7 @@
 #include "radius.cuh"
 #include "adjoint.cuh"
 #include "crp_host.h"
+#include "launch_shapes.h"
 #include "sim3d.h"
 
 namespace crp {
@@ -1458,6 +1459,7 @@ struct Sim {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int device = 0;  // the device current at crp_create
+  int sms = 1;     // its SMs
   std::string err;
 
   // Device memory: one allocation carved into aligned pieces.
@@ -1659,6 +1661,7 @@ struct Sim {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(CRP_ERR_NO_DEVICE, "no CUDA device");
     CRP_CUDA(cudaGetDevice(&device));
+    CRP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     if (user_stream) {
       stream = (cudaStream_t)user_stream;
     } else {
@@ -1690,9 +1693,7 @@ struct Sim {
     focus.control_x = gp.ctl_x;
     focus.control_y = gp.ctl_y;
     {
-      int dev = 0, sms = 0, per_sm = 0;
-      CRP_CUDA(cudaGetDevice(&dev));
-      CRP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      int per_sm = 0;
       CRP_CUDA(mixed ? radius_occupancy<PrecMixed>(&per_sm, true) : radius_occupancy<PrecFP64>(&per_sm, true));
       rp_grid_tight = std::max(1, std::min(sms * std::max(per_sm, 1), (hs.nb + kRpThreads - 1) / kRpThreads));
       CRP_CUDA(mixed ? radius_occupancy<PrecMixed>(&per_sm, false) : radius_occupancy<PrecFP64>(&per_sm, false));
@@ -1782,9 +1783,6 @@ struct Sim {
     for (int k = 0; k < 3; k++) ok = ok && make(&tm_fg[k], fg[k], fg_esz);
     if (!ok) return fail(CRP_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     // Tiles of kTileX x kTileY cells; a persistent grid of two blocks per SM.
-    int dev = 0, sms = 0;
-    CRP_CUDA(cudaGetDevice(&dev));
-    CRP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     tile_ntx = (f.X + kTileX - 1) / kTileX;
     tile_n = tile_ntx * ((f.Y + kTileY - 1) / kTileY);
     tile_grid = std::max(1, std::min(tile_n, 2 * sms));
@@ -2536,24 +2534,6 @@ struct Sim {
     return fail(CRP_ERR_INVALID, "unknown field");
   }
 
-  // Rows per chunk of the marching passes: of the numbers up to half the tuned one, that
-  // whose blocks take the least time in full waves of the 4 per SM that the GPU holds,
-  // a chunk's start counted as two rows.  Per FDTD pass with 2, 3, 4, 6 and 8 rows (us, the
-  // rule's choice in brackets): 600 x 701 12.8, [11.1], 12.7, 14.8, 16.1; 1001 x 1531 29.0,
-  // 27.0, [25.9], 26.1, 27.6; 1024 x 2048 with bubbles 43.7, 39.6, [40.7], 41.1, 47.0;
-  // 256 x 512 takes 11.7 with [1] and 13.0 with 2.
-  int march_rows(int strips) const {
-    const long slots = 148 * kMarchMinBlocks;
-    int best = 1;
-    long least = LONG_MAX;
-    for (int r = std::max(1, strip_rows / 2); r >= 1; r--) {
-      const long chunks = (gp.f.Y + r - 1) / r, blocks = strips * ((chunks + kMarchWarps - 1) / kMarchWarps);
-      const long t = (blocks + slots - 1) / slots * (r + 2);
-      if (t < least) least = t, best = r;
-    }
-    return best;
-  }
-
   // Per-precision launches.
   template <typename P>
   cudaError_t launch_fdtd(int nv, int np, int a, int b, int c, const double* src) {
@@ -2599,7 +2579,8 @@ struct Sim {
       int* perr = &d_scalars->pipe_err;
       e = launch(kClassFdtd, [&] { fdtd_tile<P><<<grid, block, smem, stream>>>(gp, fa, m, ntx, nt, perr); });
     } else {
-      const int strips = (gp.f.X + kMarchCols - 1) / kMarchCols, rows = march_rows(strips);
+      const int strips = (gp.f.X + kMarchCols - 1) / kMarchCols;
+      const int rows = march_rows(gp.f.Y, strips, strip_rows, kMarchWarps, sms * kMarchMinBlocks);
       const int chunks = (gp.f.Y + rows - 1) / rows;
       const int grid = strips * ((chunks + kMarchWarps - 1) / kMarchWarps);
       const FocalRecord rec = focal_rec;
@@ -3177,7 +3158,7 @@ crp_status Sim::adjoint(const crp_objective* obj, double* J, double* grad_amp, d
   for (int n = 0; n < N; n++) Jsum += Jn[n];
   if (J) *J = gp.dt * Jsum;
   // Reverse sweep: reverse step n reads frame set s and writes set s ^ 1.
-  const int strips = (X + 63) / 64, rows = march_rows(strips);
+  const int strips = (X + 63) / 64, rows = march_rows(Y, strips, strip_rows, kAdjWarps, sms * kAdjMinBlocks);
   const int grid = strips * (((Y + rows - 1) / rows + kAdjWarps - 1) / kAdjWarps);
   CRP_CUDA(launch(kClassOther, [&] { adj_force<<<rb, 256, 0, stream>>>(gp, fr[0], box, hist + (size_t)(N - 1) * cells_box); }));
   int s = 0;

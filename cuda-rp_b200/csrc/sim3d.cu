@@ -36,6 +36,7 @@
 #include "radius.cuh"
 #include "rk45.cuh"
 #include "lpt.cuh"
+#include "launch_shapes.h"
 #include "sim3d.h"
 
 namespace crp {
@@ -139,7 +140,6 @@ struct Fdtd3Args {
 // barriers per plane), 141 x 125 x 133 without bubbles 61 us (155).
 constexpr int kRows3 = 8;   // warps per block
 constexpr int kCols3 = 64;  // columns per warp
-constexpr int kPlanes3 = 16;  // planes per chunk, at most
 constexpr double kCloudShare3 = 0.25;
 
 enum March3Form { kPlain3 = 0, kEdges3 = 1, kVoid3 = 2 };  // inside; with x PML; with void fraction as well
@@ -1215,7 +1215,7 @@ struct Sim3Impl {
   BubbleParams bp{};
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  int device = 0;
+  int device = 0, sms = 1;
   bool mixed = false;
   std::string err;
   char* pool = nullptr;
@@ -1334,14 +1334,6 @@ struct Sim3Impl {
 
   crp_status create(const crp_config& c, const crp_bubbles_in* bin, void* user_stream);
   crp_status step_once();
-  // Planes per chunk of the marching passes: up to 16 (256^3: 398 us, 425 with 32, 402
-  // with 8), fewer where that would leave less than two waves of the 296 blocks that the
-  // GPU holds; blocks: of one chunk.
-  int march3_planes(long blocks) const {
-    int planes = d3::kPlanes3;
-    while (planes > 2 && blocks * ((g.f.Z + planes - 1) / planes) < 4 * 148) planes /= 2;
-    return planes;
-  }
   // Steps without bubbles, queued back to back: `left` more follow in this call.
   // Nothing the host decides depends on their scalars; finish_plain reads those of the
   // last step (a non-finite pressure stays non-finite in the linear step).
@@ -1478,6 +1470,7 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(CRP_ERR_NO_DEVICE, "no CUDA device");
   C3(cudaGetDevice(&device));
+  C3(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   if (user_stream) {
     stream = (cudaStream_t)user_stream;
   } else {
@@ -1681,8 +1674,6 @@ crp_status Sim3Impl::create(const crp_config& c, const crp_bubbles_in* bin, void
     C3(cudaMemcpyAsync(fg[fg_c], fg[fg_a], bytes, cudaMemcpyDeviceToDevice, stream));
     for (int q = 0; q < 3; q++) std::memcpy(supp[q], box, sizeof(box));
   }
-  int sms = 0;
-  C3(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   for (int tight = 0; tight < 2; tight++) {
     int per_sm = 0;
     if (mixed)
@@ -1779,7 +1770,7 @@ crp_status Sim3Impl::launch_fdtd(const double* elem) {
   a.oldest = (int)oldest();
   a.elem_p = elem;
   const int sx = (g.f.X + d3::kCols3 - 1) / d3::kCols3, sy = (g.f.Y + d3::kRows3 - 1) / d3::kRows3;
-  const int planes = march3_planes(sx * sy);
+  const int planes = march3_planes(g.f.Z, (long)sx * sy, sms);
   const dim3 block(32, d3::kRows3), grid(sx, sy, (g.f.Z + planes - 1) / planes);
   int u[6], w[6];
   box_union(w, supp[0], supp[1]);
@@ -2157,7 +2148,7 @@ crp_status Sim3Impl::adjoint(const crp_objective* obj, double* J, double* grad_a
   if (J) *J = g.dt * Jsum;
   // Reverse sweep: reverse step n reads frame set s and writes set s ^ 1.
   const int sx = (f.X + d3::kCols3 - 1) / d3::kCols3, sy = (f.Y + d3::kRows3 - 1) / d3::kRows3;
-  const int planes = march3_planes(sx * sy);
+  const int planes = march3_planes(g.f.Z, (long)sx * sy, sms);
   const dim3 sblk(32, d3::kRows3), sgrid(sx, sy, (f.Z + planes - 1) / planes);
   const int sb = (ns + 63) / 64;
   const double two_dt = 2.0 * g.dt;
