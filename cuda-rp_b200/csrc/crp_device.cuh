@@ -12,8 +12,6 @@
 // exactly the value MixturePropertiesKernel stores
 // (inc/bubble_CUDA_kernel.cuh:1122), so neither p0 nor rho_m occupies HBM.
 #pragma once
-#include <cuda_pipeline.h>
-
 #include <cmath>
 #include <cstdint>
 
@@ -234,12 +232,7 @@ struct F64 {
   }
   // The value get() returns after put(v).
   __device__ static __forceinline__ double stored(double v) { return v; }
-  // Asynchronous copy of element k into an 8-byte shared-memory slot, and the
-  // value of a slot once the copy has landed.
-  template <typename K>
-  __device__ __forceinline__ void stage(void* dst, K k) const {
-    __pipeline_memcpy_async(dst, p + k, 8);
-  }
+  // The value of an element copied into shared memory.
   __device__ static __forceinline__ double staged(const void* src) { return *(const double*)src; }
 };
 struct F32c {
@@ -266,10 +259,6 @@ struct F32c {
     const float h = (float)v;
     return (double)h + (double)(float)(v - (double)h);
   }
-  template <typename K>
-  __device__ __forceinline__ void stage(void* dst, K k) const {
-    __pipeline_memcpy_async(dst, p + k, 8);
-  }
   __device__ static __forceinline__ double staged(const void* src) {
     const float2 v = *(const float2*)src;
     return (double)v.x + (double)v.y;
@@ -294,10 +283,6 @@ struct F32 {
     *reinterpret_cast<float2*>(p + k) = make_float2((float)v, (float)w);
   }
   __device__ static __forceinline__ double stored(double v) { return (double)(float)v; }
-  template <typename K>
-  __device__ __forceinline__ void stage(void* dst, K k) const {
-    __pipeline_memcpy_async(dst, p + k, 4);
-  }
   __device__ static __forceinline__ double staged(const void* src) { return (double)*(const float*)src; }
 };
 
@@ -364,10 +349,6 @@ __device__ __forceinline__ Cx<R> rdiv(R a, Cx<R> b) {
 template <typename R>
 __device__ __forceinline__ Cx<R> cscl(Cx<R> a, R s) {
   return {a.re * s, a.im * s};
-}
-template <typename R>
-__device__ __forceinline__ R cabsx(Cx<R> a) {
-  return sqrt(a.re * a.re + a.im * a.im);
 }
 // cabs(a) > 0.1, decided on |a|^2 (see BubbleParams::abs2_cut64).
 template <typename R>

@@ -39,7 +39,6 @@ struct FocalRecord {
   double* out;  // null: nowhere
 };
 
-template <typename P>
 struct MarchRow {
   double2 x, y;           // px, py of the lane's two columns
   double xl, yl, xr, yr;  // and of the columns to the left and right
@@ -59,8 +58,8 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
   const bool two = i + 1 <= X;
   const bool src_rows = GEN && g.source_row > 0 && src_pressure(g);
   const unsigned pitch = (unsigned)f.pitch;
-  auto load = [&](unsigned k) -> MarchRow<P> {
-    MarchRow<P> r;
+  auto load = [&](unsigned k) -> MarchRow {
+    MarchRow r;
     r.x = a.pnx.get2(k);
     r.y = a.pny.get2(k);
     r.xl = a.pnx.get(k - 1);
@@ -71,7 +70,7 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
   };
   // p0 of columns i - 1 .. i + 2 of an interior row j, with the boundary values of
   // MixtureBoundaryPressureKernel (p0_at): the source row, then the x ghost columns.
-  auto pressures = [&](const MarchRow<P>& r, int j, double* q) {
+  auto pressures = [&](const MarchRow& r, int j, double* q) {
     q[0] = r.xl + r.yl;
     q[1] = r.x.x + r.y.x;
     q[2] = r.x.y + r.y.y;
@@ -116,7 +115,7 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
     return v;
   };
   unsigned k = (unsigned)j0 * pitch + (unsigned)(i + 1);  // row j0 - 1
-  MarchRow<P> cur = load(k);
+  MarchRow cur = load(k);
   const double2 vyb = a.vy_old.get2(k);
   double pb[4], pc[4], rb[2], rc[4], fc[2];
   pressures(cur, j0 - 1, pb);
@@ -173,7 +172,7 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
   }
   const bool wall_w = i == 1 && !g.pml_x0;
   const bool wall_m = i == X && !g.pml_x1, wall_e = i + 1 == X && !g.pml_x1;
-  MarchRow<P> nxt = load(k + pitch);
+  MarchRow nxt = load(k + pitch);
   double2 vx2 = a.vx_old.get2(k), vy2 = a.vy_old.get2(k);
   double vxl = a.vx_old.get(k - 1);
   // f_g of the row above, f_gn and f_gm of this row, one row ahead as well.
@@ -194,7 +193,7 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
     // those of one row further are requested now.
     const double2 vxo = vx2, vyo = vy2;
     const double vxw = vxl;
-    const MarchRow<P> up = nxt;
+    const MarchRow up = nxt;
     if (j < j1) {
       nxt = load(k + 2 * pitch);
       vx2 = a.vx_old.get2(k + pitch);

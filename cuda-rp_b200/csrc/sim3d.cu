@@ -144,7 +144,6 @@ constexpr double kCloudShare3 = 0.25;
 
 enum March3Form { kPlain3 = 0, kEdges3 = 1, kVoid3 = 2 };  // inside; with x PML; with void fraction as well
 
-template <typename S>
 struct Three {
   double2 x, y, z;
   __device__ __forceinline__ double2 sum() const { return make_double2(x.x + y.x + z.x, x.y + y.y + z.y); }
@@ -179,7 +178,7 @@ __device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const
   const Frame3& f = g.f;
   const bool two = i + 1 <= f.X;
   const unsigned pitch = (unsigned)f.pitch, plane = (unsigned)(f.Y + 4) * pitch;
-  auto own = [&](unsigned q) -> Three<S> { return {a.pnx.get2(q), a.pny.get2(q), a.pnz.get2(q)}; };
+  auto own = [&](unsigned q) -> Three { return {a.pnx.get2(q), a.pny.get2(q), a.pnz.get2(q)}; };
   auto one = [&](unsigned q) -> double { return a.pnx.get(q) + a.pny.get(q) + a.pnz.get(q); };
   auto rho_of = [&](double fa) -> double { return a.rho_const ? g.rho_inf : (1.0 - fa) * g.rho_inf; };
   // face3 with the roundings of v_old fa - q s2: the product q s2 rounded first.
@@ -194,7 +193,7 @@ __device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const
   unsigned q = ((unsigned)k0 * (unsigned)(f.Y + 4) + (unsigned)(j + 1)) * pitch + (unsigned)(i + 1);  // plane k0 - 1
   const double vayn = g.vay[j + 1], vbyn = g.vby[j + 1], vays = g.vay[j], vbys = g.vby[j];
   const double pay = g.pay[j], pby = g.pby[j];
-  Three<S> cur = own(q + plane);
+  Three cur = own(q + plane);
   double2 pc = cur.sum();
   double2 fc = make_double2(0.0, 0.0);  // f_g of this plane
   double zb[2];                         // the faces below
@@ -215,7 +214,7 @@ __device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const
     }
   }
   q += plane;  // plane k0
-  Three<S> nxt = own(q + plane);
+  Three nxt = own(q + plane);
   double2 vx2 = a.vx_old.get2(q), vy2 = a.vy_old.get2(q), vs2 = a.vy_old.get2(q - pitch), vz2 = a.vz_old.get2(q);
   double vxl = a.vx_old.get(q - 1);
   unsigned long long res = 0ull;
@@ -223,7 +222,7 @@ __device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const
   for (int k = k0; k <= k1; k++, q += plane) {
     const double2 vxo = vx2, vyo = vy2, vso = vs2, vzo = vz2;
     const double vxw = vxl;
-    const Three<S> up = nxt;
+    const Three up = nxt;
     const double2 pu = up.sum();
     // The neighbours of this plane, then what the next one needs.
     const double pl = one(q - 1), pr = one(q + 2);
@@ -1874,7 +1873,7 @@ crp_status Sim3Impl::launch_couple(bool pressure) {
   a.elem_p = elem_p;
   a.residual = &d_sc->residual;
   // The list's length is on the device: the blocks that the GPU holds stride over it.
-  const int grid = std::min(tiles.nx * tiles.ny * tiles.nz, 148 * 4);
+  const int grid = std::min(tiles.nx * tiles.ny * tiles.nz, sms * 4);
   d3::couple3<P><<<grid, dim3(32, 8), 0, stream>>>(g, a);
   C3(cudaGetLastError());
   launches++;
