@@ -87,10 +87,11 @@ __device__ __forceinline__ unsigned long long march_chunk(const GridParams& g, c
   };
   auto rho_of = [&](double fa) -> double { return a.rho_const ? g.rho_inf : (1.0 - fa) * g.rho_inf; };
   // dt / mean(rho) of a face, the same for both cells beside it and for every chunk:
-  // dt_rho, the plain forms' value, between densities of rho_inf (the quotient's last bit
-  // can differ from it).
+  // dt_rho, the plain forms' value, where the mean is rho_inf (the quotient's last bit can
+  // differ from it).
   auto face_factor = [&](double ra, double rb) -> double {
-    return ra == g.rho_inf && rb == g.rho_inf ? g.dt_rho : quotient(g.dt, (ra + rb) * 0.5);
+    const double m = (ra + rb) * 0.5, q = quotient(g.dt, m);
+    return m == g.rho_inf ? g.dt_rho : q;
   };
   auto predict = [&](unsigned k) {  // a ghost cell's prediction
     a.fgC.put(k, G::stored(3.0 * a.fgA.get(k) - 3.0 * a.fgB.get(k) + a.fgC.get(k)));

@@ -186,9 +186,11 @@ __device__ __forceinline__ unsigned long long march3_chunk(const Grid3& g, const
     return fma(v, fa, -__dmul_rn(q, (-p0a + p0b) * rh)) * fb;
   };
   // dt / mean(rho) of a face, the same for every cell that forms it: dt_rho, the plain
-  // forms' value, between densities of rho_inf (the quotient's last bit can differ from it).
+  // forms' value, where the mean is rho_inf (the quotient's last bit can differ from it).
   auto slow = [&](double ra, double rb) -> double {
-    return !VOID || (ra == g.rho_inf && rb == g.rho_inf) ? g.dt_rho : quotient(g.dt, (ra + rb) * 0.5);
+    if (!VOID) return g.dt_rho;
+    const double m = (ra + rb) * 0.5, q = quotient(g.dt, m);
+    return m == g.rho_inf ? g.dt_rho : q;
   };
   unsigned q = ((unsigned)k0 * (unsigned)(f.Y + 4) + (unsigned)(j + 1)) * pitch + (unsigned)(i + 1);  // plane k0 - 1
   const double vayn = g.vay[j + 1], vbyn = g.vby[j + 1], vays = g.vay[j], vbys = g.vby[j];
