@@ -129,10 +129,11 @@ __device__ __forceinline__ double weighted(double a, double x, double b, double 
 // without divisions of their own and the gas pressure costs one reciprocal; and
 // the heat flux (:521-527).
 //
-// Bound by the FP64 pipe in the quiet phase (64 % busy; the launch over 262,144
+// Bound by the FP64 pipe in the quiet phase (63 % busy; the launch over 262,144
 // bubbles of 10 sub-steps takes 77 us, 178 us with the coth form) and by the latency of
-// this chain once a few bubbles are stiff (one sub-step alone on an SM: 1,080
-// cycles for w < 32, 1,450 to 1,630 above; the coth form 4,130 above).
+// this chain once a few bubbles are stiff.  Cycles per sub-step of one warp alone, for
+// w < 32, between and above 760: quiet instance 1,330, 1,710 and 1,520; TIGHT 1,250, 1,420
+// and 1,360; the coth form 4,620.
 //
 // TIGHT: for launches that end with the chains of a few stiff bubbles.  The radius
 // update runs inside the thermal model's rounds, without branches of its own, and the
